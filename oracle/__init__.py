@@ -23,6 +23,9 @@ ORACLE_SO = os.path.join(HERE, "_bin", "liboracle.so")
 REF_DIR = os.path.join(HERE, "_ref")
 # the reference sources (only present where the oracle is built from them)
 REF_SOURCES = os.environ.get("VFRAY_REF", "/root/reference")
+if not os.path.exists(os.path.join(REF_SOURCES, "vfRayKernelCPU.cc")):
+    # a directory without the sources (an empty mount point) counts as absent
+    REF_SOURCES = os.path.join(REF_SOURCES, "absent")
 
 _u8p = np.ctypeslib.ndpointer(np.uint8, flags="C_CONTIGUOUS")
 _u32p = np.ctypeslib.ndpointer(np.uint32, flags="C_CONTIGUOUS")
