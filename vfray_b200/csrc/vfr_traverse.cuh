@@ -9,18 +9,16 @@
 // written to keep lanes converged: its arithmetic is branch-free, its rare
 // exact fallbacks (psi coordinate, exp, plane re-solve) are taken in one
 // block after the fast path, and every way a step can end is a status
-// rather than an early return.  The current tet's 4 vertices live in
-// shared memory, one slot each per thread, and a per-ray map names the slot
-// of each vertex in the entry face's rotation (r_j = local vertex
-// (f + j) & 3): the three exit candidates (f+1, f+2, f+3) read r_1..r_3
-// through it, candidate i using (r_i, r_i+1, r_i+2).  Moving to the next tet
-// stores its one new vertex in the slot of the vertex left behind and
-// rewrites the map, a permutation of slot numbers where registers rotated
-// by the entry face took 48 selects per step (2.4 % faster, and no
-// spills at 3 CTAs per SM).  Once the exit face is known, a step issues its
-// two loads together: the next tet's 32-byte walk record and the one vertex
-// the next tet does not share with this one (its id is in this tet's record),
-// so one memory round trip per step.
+// rather than an early return.  The current tet's 4 vertices live in shared
+// memory, one slot each per thread, and a per-ray map of 4 bytes names the
+// slot of each vertex in the entry face's rotation (r_j = local vertex
+// (f + j) & 3): the three exit candidates (f+1, f+2, f+3) are candidate i =
+// (r_i, r_i+1, r_i+2).  Moving to the next tet stores its one new vertex in
+// the slot of the vertex left behind and permutes the map's bytes.  Once the
+// exit face is known, a step issues its two loads together: the next tet's
+// 32-byte walk record and the one vertex the next tet does not share with
+// this one (its id is in this tet's record), so one memory round trip per
+// step.
 #pragma once
 #include "vfr_jobs.cuh"
 
@@ -41,16 +39,10 @@ namespace vfr {
 // (rounded products and differences are symmetric), and its sum and slack
 // difference are the negations of the unswapped ones.  So the swap is a sign
 // flip of (c1, c2, sum - cr): applied by xor-ing the sign of cr into them.
-//
-// v2 = c - a is passed in: candidate 3's (r1 - r3) is the negation of
-// candidate 1's (r3 - r1), exact under round-to-nearest but for the sign of
-// a zero, and that sign cannot change the test: a zero v2 component only
-// changes the sign of a product that is zero, so of a sum or difference
-// that is zero; cr = 0 is skipped, and c1, c2 and the slack difference are
-// only compared with 0 and with 0x2b8cbccc, where -0 and +0 agree.
-__device__ __forceinline__ bool exit_test_v2(const float4& a, const float4& b, float v2x,
-                                             float v2y, float ox, float oy) {
+__device__ __forceinline__ bool exit_test(const float4& a, const float4& b, const float4& c,
+                                          float ox, float oy) {
   const float v1x = fsub(b.x, a.x), v1y = fsub(b.y, a.y);
+  const float v2x = fsub(c.x, a.x), v2y = fsub(c.y, a.y);
   const float cr = fsub(fmul(v1x, v2y), fmul(v1y, v2x));
   const bool skip = below_rdelta(cr);
   const float v0x = fsub(ox, a.x), v0y = fsub(oy, a.y);
@@ -62,11 +54,6 @@ __device__ __forceinline__ bool exit_test_v2(const float4& a, const float4& b, f
   const float c2s = __uint_as_float(__float_as_uint(c2) ^ sg);
   const float ds = __uint_as_float(__float_as_uint(d) ^ sg);
   return !skip && (c1s >= 0.0f) && (c2s >= 0.0f) && (ds <= __uint_as_float(0x2b8cbcccu));
-}
-
-__device__ __forceinline__ bool exit_test(const float4& a, const float4& b, const float4& c,
-                                          float ox, float oy) {
-  return exit_test_v2(a, b, fsub(c.x, a.x), fsub(c.y, a.y), ox, oy);
 }
 
 // Per-CTA copies of the small tables: the transfer function's alpha in float
@@ -97,22 +84,117 @@ constexpr uint32_t kWatchSteps = 4095;
 // only by watched iterations, so it takes no register of the step.
 __shared__ uint32_t s_watch_saved[256];
 
-// The current tet's 4 vertices, per thread, in 4 slots; a ray's map says
-// which slot holds the vertex the entry-face rotation calls j (r_j =
-// vertex (f + j) & 3).  Moving to the next tet stores the one new vertex in
-// the slot of the vertex it replaces and rewrites the map, instead of
-// permuting 16 registers with selects.
+// The current tet's 4 vertices, per thread, in 4 slots.  A ray's map has one
+// byte per vertex, in the order r_3, r_0, r_1, r_2 of the entry face's
+// rotation (r_j = vertex (f + j) & 3): the vertex opposite the entry face
+// first.  Rotating the map right by i bytes puts the exit face i's vertices
+// (r_i, r_i+1, r_i+2) in bytes 1-3 and the vertex the step leaves behind,
+// r_i+3, in byte 0; the permutation code of the walk record then reorders
+// bytes 1-3 for the next tet (perm_selector), whose new vertex takes byte
+// 0's slot.  A byte is slot << 4 | thread >> 4, the second byte of the
+// slot's offset slot * 4096 + thread * 16 in s_vtx, so one byte permutation
+// with the thread's low offset byte gives a vertex's address.  (With 2-bit
+// fields, a shift and a mask per vertex and a 64-bit table of permutations,
+// the same map cost about 20 integer instructions more per step.)
 __shared__ float4 s_vtx[4][256];
-constexpr uint32_t kIdentityMap = 0u | 1u << 2 | 2u << 4 | 3u << 6;
-__device__ __forceinline__ uint32_t slot_of(uint32_t m, uint32_t j) { return (m >> (2u * (j & 3u))) & 3u; }
-__device__ __forceinline__ float4 vtx(uint32_t slot) { return s_vtx[slot][threadIdx.x]; }
-__device__ __forceinline__ float4 vtx_xy(uint32_t slot) {
-  const float2 v = *reinterpret_cast<const float2*>(&s_vtx[slot][threadIdx.x]);
-  return make_float4(v.x, v.y, 0.0f, 0.0f);
+__device__ __forceinline__ uint32_t identity_map() {
+  return 0x20100030u + (threadIdx.x >> 4) * 0x01010101u;
+}
+__device__ __forceinline__ char* vtx_at(uint32_t map, uint32_t byte) {
+  const uint32_t low = (threadIdx.x & 15u) << 4;
+  return reinterpret_cast<char*>(s_vtx) + __byte_perm(map, low, 0x5504u | byte << 4);
+}
+__device__ __forceinline__ float4 vtx(uint32_t map, uint32_t byte) {
+  return *reinterpret_cast<const float4*>(vtx_at(map, byte));
+}
+
+// Packed pairs of floats: sm_100's two-wide float instructions, each half
+// rounded as the single operation is.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// max(|a|, |b|, |c|); min of the same, NaN if one is NaN
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {
+  float r;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3_abs(float a, float b, float c) {
+  float r;
+  asm("min.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// The exit face of the step from rotated vertices (bytes of the map): the
+// i in 1..3 of the first candidate (r_i, r_i+1, r_i+2) the exit test accepts
+// (:310-350), 0 if none does.
+static __device__ __noinline__ uint32_t exit_face_exact(uint32_t map, float ox, float oy) {
+  const float4 r3 = vtx(map, 0), r0 = vtx(map, 1), r1 = vtx(map, 2), r2 = vtx(map, 3);
+  return exit_test(r1, r2, r3, ox, oy)   ? 1u
+         : exit_test(r2, r3, r0, ox, oy) ? 2u
+         : exit_test(r3, r0, r1, ox, oy) ? 3u
+                                         : 0u;
+}
+
+// The same from the signs of the six cross products of the vertices' offsets
+// from the ray, A_j = r_j - o: x_ab = A_a x A_b.  In real arithmetic a
+// candidate (a, b, c) has c1 = x_ab, c2 = x_ca, cr - c1 - c2 = x_bc, so the
+// ray lies inside it when the three have one sign.  With M the largest
+// component of the A_j and u = 2^-24, a computed cross product is within
+// 6.1 u M^2 of the real one, and the exit test's own c1, c2, cr and slack
+// difference (differences of vertices, at most 2M, each rounded) are within
+// 16, 16, 32 and 80 u M^2 of theirs.  So when all six products exceed
+// 2^-17 M^2 + 2e-12 = 128 u M^2 + 2e-12 in magnitude, each of them and each
+// of the test's quantities has its real sign, the slack difference is on its
+// side of 1e-12, an accepted candidate's cr is above RDELTA, and a candidate
+// is accepted exactly when its three products have one sign: of two products
+// of different sign, one fails the test whatever cr's sign is.  When the
+// entry face (r_0, r_1, r_2) holds the ray too, exactly one candidate does:
+// the ray is strictly inside it, and -A_3 lies in one of the three sectors
+// the A_j cut the plane into.  sure says that all this holds (NaN and
+// infinite coordinates fail it); about one step in 2^13 is not sure and
+// takes the exact tests.
+//
+// 40 instructions instead of 66 for three exact tests, with the six
+// products shared between the candidates.
+__device__ __forceinline__ uint32_t exit_face(uint32_t map, float ox, float oy, bool& sure) {
+  const f32x2 o = pack2(ox, oy);
+  float a0x, a0y, a1x, a1y, a2x, a2y, a3x, a3y;
+  unpack2(sub2(*reinterpret_cast<const f32x2*>(vtx_at(map, 1)), o), a0x, a0y);
+  unpack2(sub2(*reinterpret_cast<const f32x2*>(vtx_at(map, 2)), o), a1x, a1y);
+  unpack2(sub2(*reinterpret_cast<const f32x2*>(vtx_at(map, 3)), o), a2x, a2y);
+  unpack2(sub2(*reinterpret_cast<const f32x2*>(vtx_at(map, 0)), o), a3x, a3y);
+  auto cross = [](float ax, float ay, float bx, float by) {
+    return __fmaf_rn(ax, by, -fmul(ay, bx));
+  };
+  const float x01 = cross(a0x, a0y, a1x, a1y), x02 = cross(a0x, a0y, a2x, a2y);
+  const float x12 = cross(a1x, a1y, a2x, a2y), x03 = cross(a0x, a0y, a3x, a3y);
+  const float x13 = cross(a1x, a1y, a3x, a3y), x23 = cross(a2x, a2y, a3x, a3y);
+  const float M = max3_abs(max3_abs(a0x, a0y, a1x), max3_abs(a1y, a2x, a2y), max3_abs(a3x, a3y, 0.0f));
+  const float least = min3_abs(min3_abs(x01, x02, x12), min3_abs(x03, x13, x23), x23);
+  // sign bits: 01, 12, 20 alike (x20 = -x02); 12, 23, 31 alike; 23, 30, 02 alike
+  const uint32_t b01 = __float_as_uint(x01), b02 = __float_as_uint(x02), b12 = __float_as_uint(x12);
+  const uint32_t b03 = __float_as_uint(x03), b13 = __float_as_uint(x13), b23 = __float_as_uint(x23);
+  const int entry = (int)(~(b01 ^ b12) & (b12 ^ b02));
+  const int in1 = (int)(~(b12 ^ b23) & (b23 ^ b13));
+  const int in2 = (int)(~(b23 ^ b02) & (b23 ^ b03));
+  sure = least > __fmaf_rn(fmul(M, M), 0x1p-17f, 2e-12f) && entry < 0;
+  return in1 < 0 ? 1u : (in2 < 0 ? 2u : 3u);
 }
 
 struct Ray {
-  uint32_t map;                // slot of rotated vertex j in s_vtx: bits 2j..2j+1
+  uint32_t map;                // slots of the rotated vertices in s_vtx, a byte each
   WalkRec w;                   // walk record of the current tet
   const WalkRec* walk;         // this job's mesh and view vertices
   const float4* vert;
@@ -160,7 +242,7 @@ __device__ __forceinline__ bool begin_segment_at(const JobDev& J, Ray& R, uint32
   s_vtx[1][threadIdx.x] = __ldg(R.vert + sel4(id, (f + 1) & 3u));
   s_vtx[2][threadIdx.x] = __ldg(R.vert + sel4(id, (f + 2) & 3u));
   s_vtx[3][threadIdx.x] = __ldg(R.vert + sel4(id, (f + 3) & 3u));
-  R.map = kIdentityMap;
+  R.map = identity_map();
   R.zp = zp;
   R.lastZ = zp;
   R.cbi = cbi;
@@ -316,14 +398,9 @@ __device__ __forceinline__ uint32_t step(const TraverseParams& P, const SharedTa
   ++R.iters;
   const uint32_t wst = kWatched ? watched_step(P, R) : (uint32_t)kContinue;
   bool end = wst != kContinue;
-  const uint32_t m = R.map;
-  const float4 r0 = vtx_xy(slot_of(m, 0)), r1 = vtx_xy(slot_of(m, 1)), r2 = vtx_xy(slot_of(m, 2)),
-               r3 = vtx_xy(slot_of(m, 3));
-  const float e13x = fsub(r3.x, r1.x), e13y = fsub(r3.y, r1.y);
-  const bool h1 = exit_test_v2(r1, r2, e13x, e13y, R.ox, R.oy);
-  const bool h2 = exit_test(r2, r3, r0, R.ox, R.oy);
-  const bool h3 = exit_test_v2(r3, r0, -e13x, -e13y, R.ox, R.oy);
-  const uint32_t i = h1 ? 1u : (h2 ? 2u : (h3 ? 3u : 0u));
+  bool sure;
+  uint32_t i = exit_face(R.map, R.ox, R.oy, sure);
+  if (!sure) i = exit_face_exact(R.map, R.ox, R.oy);
   end = end || i == 0;  // :353 no exit face
   const uint32_t ex = (R.f + i) & 3u;
   const bool xo = (ex & 1u) != 0u, xh = (ex & 2u) != 0u;
@@ -343,8 +420,10 @@ __device__ __forceinline__ uint32_t step(const TraverseParams& P, const SharedTa
     N = ldg_walk(R.walk, tn);
     nv = __ldg(R.vert + (q & 0x07ffffffu));
   }
-  // exit face (ex, ex+1, ex+2) = (r_i, r_i+1, r_i+2)
-  const float4 a = vtx(slot_of(m, i)), b = vtx(slot_of(m, i + 1u)), c = vtx(slot_of(m, i + 2u));
+  // exit face (ex, ex+1, ex+2) = (r_i, r_i+1, r_i+2): bytes 1-3 of the
+  // rotated map
+  const uint32_t m = __funnelshift_r(R.map, R.map, 8u * i);
+  const float4 a = vtx(m, 1), b = vtx(m, 2), c = vtx(m, 3);
   // fast path: every quantity from its branch-free estimate, with a flag
   // where the estimate may differ from the reference's value
   Plane nf;
@@ -383,22 +462,14 @@ __device__ __forceinline__ uint32_t step(const TraverseParams& P, const SharedTa
     R.cbi = tfi;
   }
   const bool go_on = !end && !leaving;  // :535
-  // advance to tn through its face fn: slots fn..fn+2 are the exit face's
-  // vertices in tn's order (permutation code), slot fn+3 is the loaded
-  // vertex.  Done whatever the status: once a ray's segment ends, nothing
+  // advance to tn through its face fn: the exit face's vertices in tn's order
+  // (permutation code), the loaded vertex in the slot of the one left
+  // behind.  Done whatever the status: once a ray's segment ends, nothing
   // reads its walk state before begin_segment sets it again.
-  const uint32_t fn = (q >> 27) & 3u, code = q >> 29;
-  {
-    // the exit face's vertices are rotated i, i + 1, i + 2; slot fn + k of
-    // the next tet holds the one the permutation code names, and the new
-    // vertex takes the slot of the one left behind (rotated i + 3)
-    const uint32_t pc = perm_code(code);
-    const uint32_t s0 = slot_of(m, i + (pc & 3u)), s1 = slot_of(m, i + ((pc >> 2) & 3u));
-    const uint32_t s2 = slot_of(m, i + ((pc >> 4) & 3u)), sd = slot_of(m, i + 3u);
-    s_vtx[sd][threadIdx.x] = nv;
-    R.map = s0 | (s1 << 2) | (s2 << 4) | (sd << 6);
-  }
-  if (go_on && code >= 6) {
+  const uint32_t fn = (q >> 27) & 3u;
+  *reinterpret_cast<float4*>(vtx_at(m, 0)) = nv;
+  R.map = __byte_perm(m, 0u, perm_selector(q >> 29));
+  if (go_on && (q & 0x60000000u) == 0u) {  // kCodeMismatch: no boundary face goes on
     // shared face not matched by vertex ids: reload the tet's vertices
     const uint4 id = __ldg((kServe ? R.jp->tet : P.jobs[R.j].tet) + tn);
     bad = id_bad(id.x, R.nV) || id_bad(id.y, R.nV) || id_bad(id.z, R.nV) || id_bad(id.w, R.nV);
@@ -407,7 +478,7 @@ __device__ __forceinline__ uint32_t step(const TraverseParams& P, const SharedTa
       s_vtx[1][threadIdx.x] = __ldg(R.vert + sel4(id, (fn + 1) & 3u));
       s_vtx[2][threadIdx.x] = __ldg(R.vert + sel4(id, (fn + 2) & 3u));
       s_vtx[3][threadIdx.x] = __ldg(R.vert + sel4(id, (fn + 3) & 3u));
-      R.map = kIdentityMap;
+      R.map = identity_map();
     }
   }
   R.w = N;

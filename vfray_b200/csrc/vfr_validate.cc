@@ -64,7 +64,6 @@ namespace vfr {
 // neighbour orders the shared face's vertices relative to this tet.
 bool build_walk(const uint32_t* tet, const uint32_t* con, uint32_t nV, uint32_t nT,
                 uint32_t* walk8, std::string& why) {
-  static const int P[6][3] = {{0, 1, 2}, {0, 2, 1}, {1, 0, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}};
   if (nV > (1u << 27)) {
     why = "more than 2^27 vertices";
     return false;
@@ -75,7 +74,7 @@ bool build_walk(const uint32_t* tet, const uint32_t* con, uint32_t nV, uint32_t 
       const uint32_t n = con[4 * t + f];
       w[f] = n;
       if (n == t) {
-        w[4 + f] = 7u << 29;
+        w[4 + f] = 0u;
         continue;
       }
       const uint32_t* cn = con + 4 * (size_t)n;
@@ -95,10 +94,8 @@ bool build_walk(const uint32_t* tet, const uint32_t* con, uint32_t nV, uint32_t 
           if (tt[(f + k) & 3] == id) m[j] = k;
         ok = ok && m[j] >= 0;
       }
-      uint32_t code = 6;  // shared face not matched by ids: the walk reloads the tet
-      if (ok)
-        for (uint32_t k = 0; k < 6; ++k)
-          if (P[k][0] == m[0] && P[k][1] == m[1] && P[k][2] == m[2]) code = k;
+      uint32_t code = ok ? perm_code((uint32_t)m[0], (uint32_t)m[1], (uint32_t)m[2]) : 0u;
+      if (code == 0u) code = kCodeMismatch;  // not matched by ids: the walk reloads the tet
       w[4 + f] = tn[(fn + 3) & 3] | (fn << 27) | (code << 29);
     }
   }
