@@ -77,3 +77,18 @@ def test_batch_job_keeps_its_output_tensors():
     del j
     gc.collect()
     assert ref() is None
+
+
+def test_buffer_kept_when_a_second_waiter_is_refused():
+    s = _server([_lib.VFR_ERR_STATE, _lib.VFR_OK])
+    out = np.empty((4, 4, 3), np.uint8)
+    ref = weakref.ref(out)
+    s._outs[5] = out
+    del out
+    with pytest.raises(_lib.VfrError) as e:
+        s.wait(5)  # refused: another waiter holds the ticket, the image is still to be written
+    assert e.value.status == _lib.VFR_ERR_STATE
+    gc.collect()
+    assert ref() is not None and 5 in s._outs
+    img, _ = s.wait(5)
+    assert img is ref() and 5 not in s._outs

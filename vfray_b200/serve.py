@@ -49,10 +49,11 @@ class Server:
         """(image, info) of a request; raises VfrError on its status."""
         info = RequestInfo()
         rc = self.lib.vfr_server_wait(self.h, ticket, timeout_ms, C.byref(info))
-        # after a timeout the request is still in flight and the server will
-        # write its image later: its buffer stays referenced until a wait
-        # that returns the request's own status
-        if rc == _lib.VFR_ERR_TIMEOUT:
+        # after a timeout, or when another waiter holds the ticket
+        # (VFR_ERR_STATE), the request may still be in flight and the server
+        # will write its image later: its buffer stays referenced until the
+        # wait that returns the request's own status
+        if rc in (_lib.VFR_ERR_TIMEOUT, _lib.VFR_ERR_STATE):
             out = self._outs.get(ticket)
         else:
             out = self._outs.pop(ticket, None)
