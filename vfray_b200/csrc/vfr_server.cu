@@ -131,7 +131,7 @@ struct Seg {
   uint32_t seq = 0;     // entry of the segment table (in this epoch)
   uint32_t id = 0;      // over the server's life
   std::unique_ptr<Batch> b;
-  std::vector<Req*> reqs;
+  std::vector<Req*> reqs;  // null once done: a done request belongs to its waiter
   uint32_t remaining = 0;
   char* up = nullptr;  // pinned staging of its job-table upload
   size_t up_bytes = 0;
@@ -361,7 +361,8 @@ void vfr_server::fail_all(int rc) {
   for (Req* q : pending) finish(q);
   pending.clear();
   for (Seg* s : inflight)
-    for (Req* q : s->reqs) finish(q);
+    for (Req* q : s->reqs)
+      if (q) finish(q);
   cv_done.notify_all();
 }
 
@@ -374,7 +375,9 @@ bool vfr_server::poll_completions() {
   bool progress = false;
   const volatile uint32_t* f = flags;
   for (Seg* g : inflight)
-    for (Req* q : g->reqs) {
+    for (Req*& slot : g->reqs) {
+      Req* const q = slot;
+      if (!q) continue;
       if (q->state == St::InFlight && f[q->flag]) {
         const JobSpec& sp = g->b->specs[q->job];
         const size_t img = 3 * (size_t)sp.W * sp.H;
@@ -426,6 +429,7 @@ bool vfr_server::poll_completions() {
         steps += k.steps;
         ++completed;
         --g->remaining;
+        slot = nullptr;  // its waiter deletes the request once the lock is released
         cv_done.notify_all();
         progress = true;
       }
