@@ -504,6 +504,7 @@ int Batch::enqueue_c() {
   P.e2tab = reinterpret_cast<const double*>(C.d_tf + 256);
   P.step_cap = C.step_cap;
   P.refill = C.tune.refill;
+  P.neg0 = 0x8000000080000000ull;
   const int blocks = C.num_sms * C.traverse_blocks_per_sm(mode);
   void* args[] = {&P};
   return C.cuda(cudaLaunchKernel(C.traverse_fn(mode, C.tune.variant), dim3(blocks), dim3(256), args,

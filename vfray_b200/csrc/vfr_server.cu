@@ -301,6 +301,7 @@ int vfr_server::launch_drain() {
   SP.T.e2tab = reinterpret_cast<const double*>(X.d_tf + 256);
   SP.T.step_cap = X.step_cap;
   SP.T.refill = X.tune.refill;
+  SP.T.neg0 = 0x8000000080000000ull;
   SP.segs = segs;
   SP.ctl = ctl;
   SP.idle_limit = idle_limit.load();

@@ -56,15 +56,16 @@ __device__ __forceinline__ bool exit_test(const float4& a, const float4& b, cons
   return !skip && (c1s >= 0.0f) && (c2s >= 0.0f) && (ds <= __uint_as_float(0x2b8cbcccu));
 }
 
-// Per-CTA copies of the small tables: the transfer function's alpha in float
-// and its colour promoted to double (the compositing multiplies colours in
-// double, vfRayKernelCPU.cc:473-476, so the promotion is done once here), and
-// 2^(j/64), j = 0..63, for zeta_of.
+// Per-CTA copies of the small tables: the transfer function (RGBA, one
+// 16-byte read per step: the front's; the back's is the previous front's and
+// stays in registers), and 2^(-k/64), k = 0..511, for zeta_fast.  Divergent
+// shared reads are what the step must be sparing with: the L1 data pipe,
+// which serves them and the mesh loads, is its tightest resource (139
+// wavefronts per warp and step, 87 % of the pipe, with the colours as
+// doubles and alpha as three tables read for the front and for the back).
 struct SharedTables {
-  double2 rg[256];
-  double b[256];
-  float a[256];
-  double e2[64];
+  float4 tf[256];
+  double e2[kExpEntries];
 };
 
 // A ray's walk is a function of its state (tet, entry face) alone: the pixel
@@ -106,34 +107,6 @@ __device__ __forceinline__ char* vtx_at(uint32_t map, uint32_t byte) {
 }
 __device__ __forceinline__ float4 vtx(uint32_t map, uint32_t byte) {
   return *reinterpret_cast<const float4*>(vtx_at(map, byte));
-}
-
-// Packed pairs of floats: sm_100's two-wide float instructions, each half
-// rounded as the single operation is.
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-// max(|a|, |b|, |c|); min of the same, NaN if one is NaN
-__device__ __forceinline__ float max3_abs(float a, float b, float c) {
-  float r;
-  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-__device__ __forceinline__ float min3_abs(float a, float b, float c) {
-  float r;
-  asm("min.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
 }
 
 // The exit face of the step from rotated vertices (bytes of the map): the
@@ -201,8 +174,8 @@ struct Ray {
   uint32_t j, nT;
   uint32_t nV;                 // checked build: vertex ids are compared with it
   uint32_t watch;              // min(kWatchSteps, step cap): longer rays are checked
-  double rmaxEdge;             // 1 / maxEdgeLength, correctly rounded (div_by)
-  uint32_t cbi;                // colorBack: its transfer-function entry
+  float maxEdge, rmaxEdge;     // maxEdgeLength and its correctly rounded reciprocal
+  float4 cb;                   // colorBack (RGBA)
   uint32_t t, f, p, iters;
   float ox, oy, zp;
   float ar, ag, ab, tr, lastZ;
@@ -216,12 +189,15 @@ struct Ray {
 };
 
 // Read-only loads of the mesh through the non-coherent path (the arrays are
-// not written while the traversal runs).
+// not written while the traversal runs).  The record is one 32-byte load:
+// lanes in different tets cost the L1 data pipe 17 wavefronts fewer per warp
+// than two 16-byte loads of the same sector (122 -> 104 per step).
 __device__ __forceinline__ WalkRec ldg_walk(const WalkRec* w, uint32_t t) {
-  const uint4* p = reinterpret_cast<const uint4*>(w + t);
   WalkRec r;
-  r.n = __ldg(p);
-  r.q = __ldg(p + 1);
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r.n.x), "=r"(r.n.y), "=r"(r.n.z), "=r"(r.n.w), "=r"(r.q.x), "=r"(r.q.y), "=r"(r.q.z),
+        "=r"(r.q.w)
+      : "l"(w + t));
   return r;
 }
 
@@ -229,8 +205,8 @@ __device__ __forceinline__ WalkRec ldg_walk(const WalkRec* w, uint32_t t) {
 // back colour's transfer-function entry cbi (:256-279).  False (checked build
 // only): the tet or one of its vertex ids is out of range, and nothing was
 // loaded.
-__device__ __forceinline__ bool begin_segment_at(const JobDev& J, Ray& R, uint32_t t, uint32_t f,
-                                                 float zp, uint32_t cbi) {
+__device__ __forceinline__ bool begin_segment_at(const SharedTables& S, const JobDev& J, Ray& R,
+                                                 uint32_t t, uint32_t f, float zp, uint32_t cbi) {
   if (id_bad(t, J.nT)) return false;
   R.t = t;
   R.f = f;
@@ -245,7 +221,7 @@ __device__ __forceinline__ bool begin_segment_at(const JobDev& J, Ray& R, uint32
   R.map = identity_map();
   R.zp = zp;
   R.lastZ = zp;
-  R.cbi = cbi;
+  R.cb = S.tf[cbi];
   s_watch_saved[threadIdx.x] = 0xffffffffu;  // a new segment walks other states
   return true;
 }
@@ -255,7 +231,7 @@ __device__ __forceinline__ bool begin_segment_at(const JobDev& J, Ray& R, uint32
 // wrote in descending (depth, face) order, skipping entries above the depth
 // where the previous segment left the mesh.  Returns false when the list is
 // done (or, checked build only, holds an id out of range: VFR_DEV_RANGE).
-__device__ __forceinline__ bool next_entry(const TraverseParams& P, const JobDev& J, Ray& R,
+__device__ __forceinline__ bool next_entry(const SharedTables& S, const JobDev& J, Ray& R,
                                            uint32_t& status) {
   bool bad = false;
   while (R.de < R.en) {
@@ -269,7 +245,7 @@ __device__ __forceinline__ bool next_entry(const TraverseParams& P, const JobDev
     if (z > R.exitZ) continue;  // behind the ray already
     // stage (b) resolved the segment's start: tet << 2 | entry face, and the
     // back colour's transfer-function entry
-    if (begin_segment_at(J, R, q.z >> 2, q.z & 3u, z, q.w)) return true;
+    if (begin_segment_at(S, J, R, q.z >> 2, q.z & 3u, z, q.w)) return true;
     bad = true;
     break;
   }
@@ -312,27 +288,41 @@ __device__ __forceinline__ uint32_t watched_step(const TraverseParams& P, Ray& R
 
 // The step's depth difference and extinctions from the exit face's depth zn
 // and scalar sn at the pixel (:437-457): dz = |zPrev - zNext| (0 below
-// RDELTA) / maxEdgeLength, the front's transfer-function entry, tau of the
+// RDELTA) / maxEdgeLength, the front's colour and alpha, tau of the
 // front and of the back.  The step ends when sn is outside [0, 1] (:446).
+//
+// The fast form divides dz by maxEdgeLength through its reciprocal
+// (Markstein's correction, as in face_plane_pairs): dz is 0 or at least
+// 1e-12 and maxEdgeLength between 2^-100 and 2^80 (another one gets a NaN
+// reciprocal in start_ray, and a dz that overflows gives NaN, both of which
+// fail the psi coordinates' certificate), so nothing underflows.  Its
+// transfer-function entry (uint)(255 sn) (:452) is read off the truncated
+// sum with 2^23, and any sn indexes the table in range.
+template <bool kExact>
 __device__ __forceinline__ void extinction(const SharedTables& S, const Ray& R, float zn, float sn,
-                                           bool& end, uint32_t& tfi, float& taux,
+                                           float maxEdge, bool& end, float4& front, float& taux,
                                            float& tauy) {
-  float dz = fsub(R.zp, zn);
-  dz = dz < 0.0f ? -dz : dz;
+  float dz = fabsf(fsub(R.zp, zn));
   dz = below_rdelta(dz) ? 0.0f : dz;
   end = end || (sn < 0.0f) || (sn > 1.0f);
-  // dz /= maxEdgeLength (:450): dz is 0 or at least 1e-12 and maxEdgeLength
-  // below 2^80 (checked at upload; view set-up gives at most 2 sqrt 3), so
-  // the quotient is never subnormal and div_by is exact
-  dz = div_by(dz, R.rmaxEdge);
-  tfi = min((uint32_t)fmul(255.0f, sn), 255u);  // colorFront (:452)
-  taux = fmul(S.a[tfi], dz);
-  tauy = fmul(S.a[R.cbi], dz);
+  const float v = fmul(255.0f, sn);
+  uint32_t tfi;
+  if (kExact) {
+    dz = fdiv(dz, maxEdge);
+    tfi = min((uint32_t)v, 255u);
+  } else {
+    const float q0 = fmul(dz, R.rmaxEdge);
+    dz = __fmaf_rn(__fmaf_rn(-maxEdge, q0, dz), R.rmaxEdge, q0);
+    tfi = __float_as_uint(__fadd_rz(v, 0x1p23f)) & 255u;
+  }
+  front = S.tf[tfi];
+  taux = fmul(front.w, dz);
+  tauy = fmul(R.cb.w, dz);
 }
 
 // zeta's argument -(tau_f*0.5 + tau_b*0.5), in double (:459).  Halving is
 // exact and commutes with rounding (a double sum of two floats is never
-// subnormal), so it is the sum times -0.5: one multiplication fewer.
+// subnormal), so it is the sum times -0.5.
 __device__ __forceinline__ double zeta_arg(float taux, float tauy) {
   return dmul(dadd((double)taux, (double)tauy), -0.5);
 }
@@ -341,40 +331,44 @@ struct StepColour {
   float r, g, b, t;
 };
 
-// The step's colour and transparency (:461-483) from the front's
-// transfer-function entry, zeta and the psi coordinates (any of -1..511:
-// the table is indexed in range whatever they are).  kUnitZeta: zeta is
-// known to lie in [0, 1] (the fast path's certified zeta), which lets
-// 1 - a be formed without a conversion.
-template <bool kUnitZeta>
-__device__ __forceinline__ StepColour composite(const TraverseParams& P, const SharedTables& S,
-                                               const Ray& R, uint32_t tfi, float zeta, int ci,
-                                               int cj) {
-  const double psi = (double)__ldg(P.psi + (uint32_t)max(ci, 0) * 512u + (uint32_t)max(cj, 0));
-  const double dzeta = (double)zeta;
-  const double ca = dsub(1.0, psi), cbk = dsub(psi, dzeta);
-  const double2 frg = S.rg[tfi], brg = S.rg[R.cbi];
-  const double fbl = S.b[tfi], bbl = S.b[R.cbi];
-  const float fr = (float)dadd(dmul(frg.x, ca), dmul(brg.x, cbk));
-  const float fg = (float)dadd(dmul(frg.y, ca), dmul(brg.y, cbk));
-  const float fb = (float)dadd(dmul(fbl, ca), dmul(bbl, cbk));
-  // keep = 1 - a with a = (float)(1.0 - zeta) (innocuous double rounding);
-  // 1 - a is exact.  For zeta in [0, 1], a is 1 - zeta exactly when
-  // zeta >= 0.5 and otherwise 1 - zeta rounded to the 2^-24 grid of the
-  // floats in [0.5, 1]; either way 1 - a is zeta rounded to a multiple of
-  // 2^-24, ties to even, which adding and removing 1.5 * 2^28 in double
-  // gives.
-  double keep;
-  if (kUnitZeta) {
-    keep = dsub(dadd(dzeta, 0x1.8p28), 0x1.8p28);
-  } else {
-    const float fw = fsub(1.0f, zeta);
-    keep = dsub(1.0, (double)fw);
-  }
+// The segment's own colour (:473-476): front (1 - psi) + back (psi - zeta),
+// in double, per channel rounded to float.
+__device__ __forceinline__ float3 segment_colour(const Ray& R, const float4& front, float psif,
+                                                 float zeta) {
+  const double psi = (double)psif;
+  const double ca = dsub(1.0, psi), cbk = dsub(psi, (double)zeta);
+  return make_float3((float)dadd(dmul((double)front.x, ca), dmul((double)R.cb.x, cbk)),
+                     (float)dadd(dmul((double)front.y, ca), dmul((double)R.cb.y, cbk)),
+                     (float)dadd(dmul((double)front.z, ca), dmul((double)R.cb.z, cbk)));
+}
+
+// The step's colour and transparency (:477-483) as the reference computes
+// them: keep = 1 - a in double with a = (float)(1.0 - zeta).
+__device__ __forceinline__ StepColour composite_exact(const Ray& R, float3 f, float zeta) {
+  const double keep = dsub(1.0, (double)fsub(1.0f, zeta));
   StepColour o;
-  o.r = (float)dadd((double)fr, dmul(keep, (double)R.ar));
-  o.g = (float)dadd((double)fg, dmul(keep, (double)R.ag));
-  o.b = (float)dadd((double)fb, dmul(keep, (double)R.ab));
+  o.r = (float)dadd((double)f.x, dmul(keep, (double)R.ar));
+  o.g = (float)dadd((double)f.y, dmul(keep, (double)R.ag));
+  o.b = (float)dadd((double)f.z, dmul(keep, (double)R.ab));
+  o.t = fmul(R.tr, zeta);
+  return o;
+}
+
+// The same for zeta in [0, 1].  1 - a is then a float: zeta rounded to a
+// multiple of 2^-24 (exact in float: a is 1 - zeta or a multiple of 2^-24),
+// its product with a float is exact in double, and the reference's result is
+// that sum rounded to double and then to float.  One FMA rounds it once: the
+// two differ only where the double rounding lands on a midpoint between
+// floats, which takes a sum of more than 53 bits (the accumulated channel
+// below a 32nd of the new one) and 28 equal bits in a row, and there the FMA
+// is the one nearer to the exact sum.  3 instructions instead of 15, 9 of
+// them conversions.
+__device__ __forceinline__ StepColour composite_fast(const Ray& R, float3 f, float zeta) {
+  const float keep = fsub(1.0f, fsub(1.0f, zeta));
+  StepColour o;
+  o.r = __fmaf_rn(keep, R.ar, f.x);
+  o.g = __fmaf_rn(keep, R.ag, f.y);
+  o.b = __fmaf_rn(keep, R.ab, f.z);
   o.t = fmul(R.tr, zeta);
   return o;
 }
@@ -426,40 +420,43 @@ __device__ __forceinline__ uint32_t step(const TraverseParams& P, const SharedTa
   const float4 a = vtx(m, 1), b = vtx(m, 2), c = vtx(m, 3);
   // fast path: every quantity from its branch-free estimate, with a flag
   // where the estimate may differ from the reference's value
-  Plane nf;
-  const bool plane_ok = face_plane_fast(a, b, c, nf);
-  float zn = plane_eval(R.ox, R.oy, nf.zx, nf.zy, nf.zz);
+  float zn, sn;
+  const bool plane_ok = face_depth_fast(a, b, c, R.ox, R.oy, P.neg0, zn, sn);
   const bool end0 = end;
-  uint32_t tfi;
+  float4 front;
   float taux, tauy;
-  extinction(S, R, zn, plane_eval(R.ox, R.oy, nf.sx, nf.sy, nf.sz), end, tfi, taux, tauy);
-  bool z_ok, i_ok, j_ok;
-  float zeta = zeta_fast(zeta_arg(taux, tauy), S.e2, z_ok);
-  int ci = psi_coord_fast(taux, i_ok), cj = psi_coord_fast(tauy, j_ok);
-  StepColour col = composite<true>(P, S, R, tfi, zeta, ci, cj);
+  extinction<false>(S, R, zn, sn, R.maxEdge, end, front, taux, tauy);
+  bool z_ok, psi_ok;
+  float zeta = zeta_fast(taux, tauy, S.e2, z_ok);
+  const uint32_t pij = psi_coords_fast(taux, tauy, psi_ok);
+  StepColour col = composite_fast(R, segment_colour(R, front, __ldg(P.psi + pij), zeta), zeta);
   // rare: the exact path for the lanes whose plane, zeta or psi coordinate
   // was not certified (a plane with a tiny coefficient; about one psi
-  // coordinate in 2^10), before anything is committed
-  if ((!plane_ok && !end0) || (!end && !(z_ok && i_ok && j_ok))) {
+  // coordinate in 2^12), before anything is committed
+  if ((!plane_ok && !end0) || (!end && !(z_ok && psi_ok))) {
     if (!plane_ok) {
+      Plane nf;
       face_plane_ieee(a, b, c, nf);
       zn = plane_eval(R.ox, R.oy, nf.zx, nf.zy, nf.zz);
-      end = end0;
-      extinction(S, R, zn, plane_eval(R.ox, R.oy, nf.sx, nf.sy, nf.sz), end, tfi, taux, tauy);
+      sn = plane_eval(R.ox, R.oy, nf.sx, nf.sy, nf.sz);
     }
-    zeta = zeta_of(zeta_arg(taux, tauy), S.e2);
-    ci = psi_coord(taux);
-    cj = psi_coord(tauy);
-    col = composite<false>(P, S, R, tfi, zeta, ci, cj);
+    end = end0;
+    extinction<true>(S, R, zn, sn, job_maxedge(kServe ? *R.jp : P.jobs[R.j]), end, front, taux,
+                     tauy);
+    zeta = zeta_fast(taux, tauy, S.e2, z_ok);
+    if (!(z_ok && taux >= 0.0f && tauy >= 0.0f)) zeta = (float)exp(zeta_arg(taux, tauy));
+    const int ci = psi_coord_double(taux), cj = psi_coord_double(tauy);
+    end = end || (ci | cj) < 0;  // :468
+    const float psi = __ldg(P.psi + (uint32_t)max(ci, 0) * 512u + (uint32_t)max(cj, 0));
+    col = composite_exact(R, segment_colour(R, front, psi, zeta), zeta);
   }
-  end = end || (ci | cj) < 0;  // :468
   if (!end) {
     R.ar = col.r;
     R.ag = col.g;
     R.ab = col.b;
     R.tr = col.t;
     R.lastZ = zn;
-    R.cbi = tfi;
+    R.cb = front;
   }
   const bool go_on = !end && !leaving;  // :535
   // advance to tn through its face fn: the exit face's vertices in tn's order
@@ -498,14 +495,16 @@ __device__ __forceinline__ uint32_t step(const TraverseParams& P, const SharedTa
 // mode; kMode 2 takes the mode from the job).  Returns whether the ray
 // walks; a composited pixel without a usable entry is finished here.
 template <int kMode>
-__device__ __forceinline__ bool start_ray(const TraverseParams& P, const JobDev& J, Ray& R,
-                                          uint32_t local, uint32_t& status) {
+__device__ __forceinline__ bool start_ray(const TraverseParams& P, const SharedTables& S,
+                                          const JobDev& J, Ray& R, uint32_t local,
+                                          uint32_t& status) {
   R.walk = J.walk;
   R.vert = J.vert;
   R.nT = J.nT;
   R.nV = J.nV;
   R.watch = min(kWatchSteps, step_cap_of(P, J.nT));
-  R.rmaxEdge = __drcp_rn((double)job_maxedge(J));
+  R.maxEdge = job_maxedge(J);
+  R.rmaxEdge = R.maxEdge >= 0x1p-100f ? __frcp_rn(R.maxEdge) : __uint_as_float(0x7fffffffu);
   const RayStart rs = J.rays[local];
   R.p = rs.p;
   if (id_bad(R.p, J.W * J.H)) {
@@ -520,7 +519,7 @@ __device__ __forceinline__ bool start_ray(const TraverseParams& P, const JobDev&
   R.iters = 0;
   const bool ref = kMode == 0 || (kMode == 2 && J.mode == 0);
   if (ref) {  // stage (b) resolved the winning face's segment start
-    if (!begin_segment_at(J, R, rs.tf >> 2, rs.tf & 3u, __uint_as_float(rs.zp), rs.cbi)) {
+    if (!begin_segment_at(S, J, R, rs.tf >> 2, rs.tf & 3u, __uint_as_float(rs.zp), rs.cbi)) {
       status |= kDevRange;
       return false;
     }
@@ -530,7 +529,7 @@ __device__ __forceinline__ bool start_ray(const TraverseParams& P, const JobDev&
   R.en = J.ent_cnt[R.p];
   R.exitZ = INFINITY;
   R.de = 0;
-  if (next_entry(P, J, R, status)) return true;
+  if (next_entry(S, J, R, status)) return true;
   finish_pixel(J, R);
   return false;
 }
@@ -556,13 +555,10 @@ __device__ __forceinline__ void flush(const TraverseParams& P, Tally& T) {
 // kMinBlocks: CTAs of 256 threads the register budget must allow per SM
 // (2: no spills; 3: 80 registers, a few spilled to L1).
 __device__ __forceinline__ void load_tables(const TraverseParams& P, SharedTables& S) {
-  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) {
-    const float4 c = P.tf[i];
-    S.rg[i] = make_double2((double)c.x, (double)c.y);
-    S.b[i] = (double)c.z;
-    S.a[i] = c.w;
-  }
-  for (uint32_t i = threadIdx.x; i < 64; i += blockDim.x) S.e2[i] = P.e2tab[i];
+  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) S.tf[i] = P.tf[i];
+  // 2^(-k/64) from the table of 2^(j/64), j = 0..63, scaled by a power of two
+  for (uint32_t k = threadIdx.x; k < kExpEntries; k += blockDim.x)
+    S.e2[k] = P.e2tab[(64u - (k & 63u)) & 63u] * (1.0 / (double)(1u << ((k + 63u) >> 6)));
   __syncthreads();
 }
 
@@ -595,7 +591,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) traverse_kernel(TraverseParam
             T.j = j;
           }
           R.j = j;
-          active = start_ray<kMode>(P, J, R, g - P.ray_pref[j], T.status);
+          active = start_ray<kMode>(P, S, J, R, g - P.ray_pref[j], T.status);
         }
       }
     }
@@ -618,7 +614,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) traverse_kernel(TraverseParam
     if (res == kSegmentEnd) {
       if (kMode == 1) {
         R.exitZ = R.lastZ;
-        if (next_entry(P, P.jobs[R.j], R, T.status)) continue;
+        if (next_entry(S, P.jobs[R.j], R, T.status)) continue;
       }
       finish_pixel(P.jobs[R.j], R);
     } else if (res == kCycle || res == kCap) {
@@ -767,7 +763,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) serve_kernel(ServeParams SP) 
           R.jp = sg.jobs + j;
           R.done = sg.done + j;
           uint32_t status = 0;
-          active = start_ray<2>(P, *R.jp, R, g - sg.ray_pref[j], status);
+          active = start_ray<2>(P, S, *R.jp, R, g - sg.ray_pref[j], status);
           if (!active) served_ray_done(R, status);
         }
       }
@@ -810,7 +806,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) serve_kernel(ServeParams SP) 
       if (res == kSegmentEnd) {
         if (R.jp->mode == 1) {
           R.exitZ = R.lastZ;
-          fin = !next_entry(P, *R.jp, R, status);
+          fin = !next_entry(S, *R.jp, R, status);
         }
         if (fin) finish_pixel(*R.jp, R);
       } else if (res == kCycle || res == kCap) {

@@ -76,6 +76,7 @@ struct TraverseParams {
   const double* e2tab;       // 2^(j/64), j = 0..63
   uint32_t step_cap;         // 0: 4 * nT + 64 of each job's mesh
   uint32_t refill;           // refill a warp's idle lanes once this many are idle
+  f32x2 neg0;                // (-0.0f, -0.0f), see face_plane_pairs
 };
 
 // ---- served form ----
