@@ -92,28 +92,50 @@ __shared__ uint32_t s_watch_saved[256];
 // (r_i, r_i+1, r_i+2) in bytes 1-3 and the vertex the step leaves behind,
 // r_i+3, in byte 0; the permutation code of the walk record then reorders
 // bytes 1-3 for the next tet (perm_selector), whose new vertex takes byte
-// 0's slot.  A byte is slot << 4 | thread >> 4, the second byte of the
-// slot's offset slot * 4096 + thread * 16 in s_vtx, so one byte permutation
-// with the thread's low offset byte gives a vertex's address.  (With 2-bit
-// fields, a shift and a mask per vertex and a 64-bit table of permutations,
-// the same map cost about 20 integer instructions more per step.)
-__shared__ float4 s_vtx[4][256];
+// 0's slot.  A byte is the second byte of the vertex's 16-bit shared-memory
+// address, slot * 4096 + thread * 16 from the 256-byte aligned start of
+// s_vtx, so one byte permutation with the thread's low address byte gives an
+// address that the load takes as it is.  (With 2-bit fields, a shift and a
+// mask per vertex and a 64-bit table of permutations, the map cost about 20
+// integer instructions more per step; with offsets into the array, which the
+// compiler adds to its base, 10 more: 8.21 -> 8.12 ms for 32 views.)
+__shared__ __align__(256) float4 s_vtx[4][256];
 __device__ __forceinline__ uint32_t identity_map() {
-  return 0x20100030u + (threadIdx.x >> 4) * 0x01010101u;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(s_vtx) >> 8;
+  return 0x20100030u + ((threadIdx.x >> 4) + base) * 0x01010101u;
 }
-__device__ __forceinline__ char* vtx_at(uint32_t map, uint32_t byte) {
-  const uint32_t low = (threadIdx.x & 15u) << 4;
-  return reinterpret_cast<char*>(s_vtx) + __byte_perm(map, low, 0x5504u | byte << 4);
+// The thread's low offset byte, held in a register rather than read from
+// the thread index at each use.
+__device__ __forceinline__ uint32_t thread_low() {
+  uint32_t low = (threadIdx.x & 15u) << 4;
+  asm volatile("" : "+r"(low));
+  return low;
 }
-__device__ __forceinline__ float4 vtx(uint32_t map, uint32_t byte) {
-  return *reinterpret_cast<const float4*>(vtx_at(map, byte));
+__device__ __forceinline__ uint32_t vtx_at(uint32_t map, uint32_t low, uint32_t byte) {
+  return __byte_perm(map, low, 0x5504u | byte << 4);
+}
+__device__ __forceinline__ float4 vtx(uint32_t at) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+  return v;
+}
+__device__ __forceinline__ f32x2 vtx_xy(uint32_t at) {
+  f32x2 v;
+  asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(at));
+  return v;
+}
+__device__ __forceinline__ void set_vtx(uint32_t at, float4 v) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(v.x), "f"(v.y), "f"(v.z),
+               "f"(v.w));
 }
 
 // The exit face of the step from rotated vertices (bytes of the map): the
 // i in 1..3 of the first candidate (r_i, r_i+1, r_i+2) the exit test accepts
 // (:310-350), 0 if none does.
-static __device__ __noinline__ uint32_t exit_face_exact(uint32_t map, float ox, float oy) {
-  const float4 r3 = vtx(map, 0), r0 = vtx(map, 1), r1 = vtx(map, 2), r2 = vtx(map, 3);
+static __device__ __noinline__ uint32_t exit_face_exact(uint32_t map, uint32_t low, float ox, float oy) {
+  const float4 r3 = vtx(vtx_at(map, low, 0)), r0 = vtx(vtx_at(map, low, 1)),
+               r1 = vtx(vtx_at(map, low, 2)), r2 = vtx(vtx_at(map, low, 3));
   return exit_test(r1, r2, r3, ox, oy)   ? 1u
          : exit_test(r2, r3, r0, ox, oy) ? 2u
          : exit_test(r3, r0, r1, ox, oy) ? 3u
@@ -141,13 +163,14 @@ static __device__ __noinline__ uint32_t exit_face_exact(uint32_t map, float ox, 
 //
 // 40 instructions instead of 66 for three exact tests, with the six
 // products shared between the candidates.
-__device__ __forceinline__ uint32_t exit_face(uint32_t map, float ox, float oy, bool& sure) {
+__device__ __forceinline__ uint32_t exit_face(uint32_t map, uint32_t low, float ox, float oy,
+                                              bool& sure) {
   const f32x2 o = pack2(ox, oy);
   float a0x, a0y, a1x, a1y, a2x, a2y, a3x, a3y;
-  unpack2(sub2(*reinterpret_cast<const f32x2*>(vtx_at(map, 1)), o), a0x, a0y);
-  unpack2(sub2(*reinterpret_cast<const f32x2*>(vtx_at(map, 2)), o), a1x, a1y);
-  unpack2(sub2(*reinterpret_cast<const f32x2*>(vtx_at(map, 3)), o), a2x, a2y);
-  unpack2(sub2(*reinterpret_cast<const f32x2*>(vtx_at(map, 0)), o), a3x, a3y);
+  unpack2(sub2(vtx_xy(vtx_at(map, low, 1)), o), a0x, a0y);
+  unpack2(sub2(vtx_xy(vtx_at(map, low, 2)), o), a1x, a1y);
+  unpack2(sub2(vtx_xy(vtx_at(map, low, 3)), o), a2x, a2y);
+  unpack2(sub2(vtx_xy(vtx_at(map, low, 0)), o), a3x, a3y);
   auto cross = [](float ax, float ay, float bx, float by) {
     return __fmaf_rn(ax, by, -fmul(ay, bx));
   };
@@ -166,8 +189,16 @@ __device__ __forceinline__ uint32_t exit_face(uint32_t map, float ox, float oy, 
   return in1 < 0 ? 1u : (in2 < 0 ? 2u : 3u);
 }
 
+// Composited mode: the pixel's entry list (first, count), the next entry to
+// take and the depth where the last segment left the mesh, in shared memory:
+// only a segment's end reads them, and the step needs the registers (spills
+// 46 -> 22 bytes at 3 CTAs per SM).
+__shared__ uint32_t s_ea[256], s_en[256], s_de[256];
+__shared__ float s_exit_z[256];
+
 struct Ray {
   uint32_t map;                // slots of the rotated vertices in s_vtx, a byte each
+  uint32_t low;                // the thread's low offset byte in a slot
   WalkRec w;                   // walk record of the current tet
   const WalkRec* walk;         // this job's mesh and view vertices
   const float4* vert;
@@ -179,9 +210,6 @@ struct Ray {
   uint32_t t, f, p, iters;
   float ox, oy, zp;
   float ar, ag, ab, tr, lastZ;
-  // composited mode: this pixel's entry list and the next entry to take
-  uint32_t ea, en, de;
-  float exitZ;
   // served form: the job (its table entry lives in the server's arena) and
   // its completion flag
   const JobDev* jp;
@@ -214,11 +242,12 @@ __device__ __forceinline__ bool begin_segment_at(const SharedTables& S, const Jo
   if (id_bad(id.x, J.nV) || id_bad(id.y, J.nV) || id_bad(id.z, J.nV) || id_bad(id.w, J.nV))
     return false;
   R.w = ldg_walk(R.walk, t);
-  s_vtx[0][threadIdx.x] = __ldg(R.vert + sel4(id, f));
-  s_vtx[1][threadIdx.x] = __ldg(R.vert + sel4(id, (f + 1) & 3u));
-  s_vtx[2][threadIdx.x] = __ldg(R.vert + sel4(id, (f + 2) & 3u));
-  s_vtx[3][threadIdx.x] = __ldg(R.vert + sel4(id, (f + 3) & 3u));
-  R.map = identity_map();
+  const uint32_t ident = identity_map();
+  set_vtx(vtx_at(ident, R.low, 1), __ldg(R.vert + sel4(id, f)));
+  set_vtx(vtx_at(ident, R.low, 2), __ldg(R.vert + sel4(id, (f + 1) & 3u)));
+  set_vtx(vtx_at(ident, R.low, 3), __ldg(R.vert + sel4(id, (f + 2) & 3u)));
+  set_vtx(vtx_at(ident, R.low, 0), __ldg(R.vert + sel4(id, (f + 3) & 3u)));
+  R.map = ident;
   R.zp = zp;
   R.lastZ = zp;
   R.cb = S.tf[cbi];
@@ -234,23 +263,28 @@ __device__ __forceinline__ bool begin_segment_at(const SharedTables& S, const Jo
 __device__ __forceinline__ bool next_entry(const SharedTables& S, const JobDev& J, Ray& R,
                                            uint32_t& status) {
   bool bad = false;
-  while (R.de < R.en) {
-    if (id_bad(R.ea + R.de, J.ent_cap)) {
+  const uint32_t ea = s_ea[threadIdx.x], en = s_en[threadIdx.x];
+  const float exit_z = s_exit_z[threadIdx.x];
+  uint32_t de = s_de[threadIdx.x];
+  bool started = false;
+  while (de < en) {
+    if (id_bad(ea + de, J.ent_cap)) {
       bad = true;
       break;
     }
-    const uint4 q = J.ent[R.ea + R.de];
-    ++R.de;
+    const uint4 q = J.ent[ea + de];
+    ++de;
     const float z = __uint_as_float(q.x);
-    if (z > R.exitZ) continue;  // behind the ray already
+    if (z > exit_z) continue;  // behind the ray already
     // stage (b) resolved the segment's start: tet << 2 | entry face, and the
     // back colour's transfer-function entry
-    if (begin_segment_at(S, J, R, q.z >> 2, q.z & 3u, z, q.w)) return true;
-    bad = true;
+    started = begin_segment_at(S, J, R, q.z >> 2, q.z & 3u, z, q.w);
+    bad = !started;
     break;
   }
+  s_de[threadIdx.x] = de;
   if (bad) status |= kDevRange;
-  return false;
+  return started;
 }
 
 __device__ __forceinline__ void finish_pixel(const JobDev& J, const Ray& R) {
@@ -393,8 +427,8 @@ __device__ __forceinline__ uint32_t step(const TraverseParams& P, const SharedTa
   const uint32_t wst = kWatched ? watched_step(P, R) : (uint32_t)kContinue;
   bool end = wst != kContinue;
   bool sure;
-  uint32_t i = exit_face(R.map, R.ox, R.oy, sure);
-  if (!sure) i = exit_face_exact(R.map, R.ox, R.oy);
+  uint32_t i = exit_face(R.map, R.low, R.ox, R.oy, sure);
+  if (!sure) i = exit_face_exact(R.map, R.low, R.ox, R.oy);
   end = end || i == 0;  // :353 no exit face
   const uint32_t ex = (R.f + i) & 3u;
   const bool xo = (ex & 1u) != 0u, xh = (ex & 2u) != 0u;
@@ -417,7 +451,8 @@ __device__ __forceinline__ uint32_t step(const TraverseParams& P, const SharedTa
   // exit face (ex, ex+1, ex+2) = (r_i, r_i+1, r_i+2): bytes 1-3 of the
   // rotated map
   const uint32_t m = __funnelshift_r(R.map, R.map, 8u * i);
-  const float4 a = vtx(m, 1), b = vtx(m, 2), c = vtx(m, 3);
+  const float4 a = vtx(vtx_at(m, R.low, 1)), b = vtx(vtx_at(m, R.low, 2)),
+               c = vtx(vtx_at(m, R.low, 3));
   // fast path: every quantity from its branch-free estimate, with a flag
   // where the estimate may differ from the reference's value
   float zn, sn;
@@ -464,18 +499,19 @@ __device__ __forceinline__ uint32_t step(const TraverseParams& P, const SharedTa
   // behind.  Done whatever the status: once a ray's segment ends, nothing
   // reads its walk state before begin_segment sets it again.
   const uint32_t fn = (q >> 27) & 3u;
-  *reinterpret_cast<float4*>(vtx_at(m, 0)) = nv;
+  set_vtx(vtx_at(m, R.low, 0), nv);
   R.map = __byte_perm(m, 0u, perm_selector(q >> 29));
   if (go_on && (q & 0x60000000u) == 0u) {  // kCodeMismatch: no boundary face goes on
     // shared face not matched by vertex ids: reload the tet's vertices
     const uint4 id = __ldg((kServe ? R.jp->tet : P.jobs[R.j].tet) + tn);
     bad = id_bad(id.x, R.nV) || id_bad(id.y, R.nV) || id_bad(id.z, R.nV) || id_bad(id.w, R.nV);
     if (!bad) {
-      s_vtx[0][threadIdx.x] = __ldg(R.vert + sel4(id, fn));
-      s_vtx[1][threadIdx.x] = __ldg(R.vert + sel4(id, (fn + 1) & 3u));
-      s_vtx[2][threadIdx.x] = __ldg(R.vert + sel4(id, (fn + 2) & 3u));
-      s_vtx[3][threadIdx.x] = __ldg(R.vert + sel4(id, (fn + 3) & 3u));
-      R.map = identity_map();
+      const uint32_t ident = identity_map();
+      set_vtx(vtx_at(ident, R.low, 1), __ldg(R.vert + sel4(id, fn)));
+      set_vtx(vtx_at(ident, R.low, 2), __ldg(R.vert + sel4(id, (fn + 1) & 3u)));
+      set_vtx(vtx_at(ident, R.low, 3), __ldg(R.vert + sel4(id, (fn + 2) & 3u)));
+      set_vtx(vtx_at(ident, R.low, 0), __ldg(R.vert + sel4(id, (fn + 3) & 3u)));
+      R.map = ident;
     }
   }
   R.w = N;
@@ -525,10 +561,10 @@ __device__ __forceinline__ bool start_ray(const TraverseParams& P, const SharedT
     }
     return true;
   }
-  R.ea = J.ent_off[R.p];
-  R.en = J.ent_cnt[R.p];
-  R.exitZ = INFINITY;
-  R.de = 0;
+  s_ea[threadIdx.x] = J.ent_off[R.p];
+  s_en[threadIdx.x] = J.ent_cnt[R.p];
+  s_exit_z[threadIdx.x] = INFINITY;
+  s_de[threadIdx.x] = 0;
   if (next_entry(S, J, R, status)) return true;
   finish_pixel(J, R);
   return false;
@@ -573,6 +609,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) traverse_kernel(TraverseParam
   Tally T = {0xffffffffu, 0ull, 0u};
   bool active = false, exhausted = false;
   Ray R;
+  R.low = thread_low();
   for (;;) {
     const uint32_t idle = __ballot_sync(0xffffffffu, !active);
     if (idle && !exhausted && ((uint32_t)__popc(idle) >= refill || idle == 0xffffffffu)) {
@@ -613,7 +650,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) traverse_kernel(TraverseParam
     if (res == kContinue) continue;
     if (res == kSegmentEnd) {
       if (kMode == 1) {
-        R.exitZ = R.lastZ;
+        s_exit_z[threadIdx.x] = R.lastZ;
         if (next_entry(S, P.jobs[R.j], R, T.status)) continue;
       }
       finish_pixel(P.jobs[R.j], R);
@@ -723,6 +760,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) serve_kernel(ServeParams SP) 
   uint32_t backoff = 256, quiet = 0;
   bool active = false;
   Ray R;
+  R.low = thread_low();
   for (;;) {
     const uint32_t idle = __ballot_sync(0xffffffffu, !active);
     uint32_t seg = 0xffffffffu;
@@ -805,7 +843,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) serve_kernel(ServeParams SP) 
       fin = true;
       if (res == kSegmentEnd) {
         if (R.jp->mode == 1) {
-          R.exitZ = R.lastZ;
+          s_exit_z[threadIdx.x] = R.lastZ;
           fin = !next_entry(S, *R.jp, R, status);
         }
         if (fin) finish_pixel(*R.jp, R);
