@@ -362,16 +362,19 @@ __global__ void __launch_bounds__(256, 4) raster_kernel(const JobDev* __restrict
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t total = vpref[njobs];
-  // A warp takes 32 consecutive visible faces at a time.  Each lane loads and
-  // sets up one of them (plane, box, entry edges: 32 independent load
-  // chains in flight instead of one), then the warp covers the faces one
+  // A warp takes up to 32 consecutive visible faces at a time.  Each lane
+  // loads and sets up one of them (plane, box, entry edges: 32 independent
+  // load chains in flight instead of one), then the warp covers the faces one
   // after another with the setup broadcast from the lane that made it
   // (1.25 -> 0.83 ms for 64 views at 512^2 against one warp per face; the
   // register bound of 4 CTAs per SM spills 20 bytes and beats the unbounded
-  // 70 registers at 3 CTAs).
-  for (uint32_t g0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32u; g0 < total;
-       g0 += nwarps * 32u) {
-    const uint32_t g = g0 + lane;
+  // 70 registers at 3 CTAs).  Covering is serial in a warp, so where there
+  // are fewer than 32 faces per launched warp -- a single view has a few
+  // thousand to a few ten thousand -- each warp takes only its share.
+  const uint32_t per = min(32u, (total + nwarps - 1u) / nwarps);
+  for (uint32_t g0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per; g0 < total;
+       g0 += nwarps * per) {
+    const uint32_t g = lane < per ? g0 + lane : total;
     bool has = false;
     uint32_t j = 0, e = 0, bx = 0, by = 0, xe = 0, ye = 0;
     EntryEdges E = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
