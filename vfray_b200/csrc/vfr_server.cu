@@ -56,6 +56,7 @@ using vfr::JobSpec;
 constexpr uint32_t kMaxSegs = 8192;        // segment-table entries per epoch
 constexpr uint32_t kMaxFlags = 1u << 20;   // completion flags per epoch
 constexpr int kReserveDivisor = 2;        // traversal CTAs left out for the preparation: SMs / this
+constexpr size_t kHandOver = 1u << 20;     // image bytes copied to a caller in one pass
 constexpr uint32_t kIdleLimit = 400000;    // default: microseconds an idle drain waits for work
 constexpr double kLingerMs = 50.0;         // default: idle time before the worker stops the drain
 
@@ -77,6 +78,7 @@ struct Req {
   uint64_t num_steps = 0;
   char* stage = nullptr;  // pinned: the image (unless copied directly), then the job's counters
   size_t stage_bytes = 0, img_off = 0;
+  size_t handed = 0;      // image bytes already in the caller's buffer
   cudaEvent_t copied = nullptr;
 };
 
@@ -412,7 +414,18 @@ bool vfr_server::poll_completions() {
         const size_t img = 3 * (size_t)sp.W * sp.H;
         vfr::ViewCounters k;
         std::memcpy(&k, q->stage + q->img_off, sizeof k);
-        if (q->r.rgb8_host && q->img_off) std::memcpy(q->r.rgb8_host, q->stage, img);
+        if (q->r.rgb8_host && q->img_off) {
+          // a large image goes to the caller a piece per pass, so that
+          // requests that arrive meanwhile are admitted between the pieces
+          // (a 2048^2 image into fresh pages takes 1.5 ms)
+          const size_t piece = std::min(img - q->handed, kHandOver);
+          std::memcpy(q->r.rgb8_host + q->handed, q->stage + q->handed, piece);
+          q->handed += piece;
+          if (q->handed < img) {
+            progress = true;
+            continue;
+          }
+        }
         pool.release(q->stage, q->stage_bytes);
         q->stage = nullptr;
         cudaEventDestroy(q->copied);
