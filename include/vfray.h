@@ -63,7 +63,7 @@ extern "C" {
 #define VFR_OPT_PROFILE 4         /* 1: record per-stage CUDA events of every view */
 #define VFR_OPT_TRAVERSE_VARIANT 5 /* traversal register budget: 0 = 2 CTAs/SM, 1 = 3 CTAs/SM (1) */
 #define VFR_OPT_REFILL 6          /* queue chunk: a warp takes rays from the work queue once at
-                                     least this many of its lanes are idle, one per idle lane (4) */
+                                     least this many of its lanes are idle, one per idle lane (7) */
 #define VFR_OPT_RASTER_WARPS 7    /* stage (b) warps per SM (64) */
 #define VFR_OPT_TILE_WIDTH 8      /* ray-list screen tile width: 4, 8, 16, 32 (4 = 4x8) */
 

@@ -70,7 +70,12 @@ struct Mesh {
 
 struct Tuning {
   uint32_t blocks_per_sm = 0;  // traversal CTAs per SM (0: occupancy maximum)
-  uint32_t refill = 4;         // refill idle lanes once this many of a warp's are idle
+  // Refill a warp's idle lanes once this many are idle: a refill stops the
+  // whole warp for a chain of dependent loads, so it pays to wait, and each
+  // idle lane loses its steps.  32 views at 512^2 of the carved 64^3 mesh at
+  // 4 / 6 / 7 / 8: 8.12 / 7.92 / 7.87 / 7.97 ms (24 composited views 3.95 /
+  // 3.78 / 3.72 / 3.73, a 2048^2 view 6.58 / 6.47 / 6.44 / 6.59).
+  uint32_t refill = 7;
   uint32_t variant = 1;        // traversal register budget: 0 = 2 CTAs/SM, 1 = 3 CTAs/SM
   uint32_t raster_warps_per_sm = 64;
   uint32_t tile_w = 4;          // ray-list tile width (x 32/tile_w rows)
