@@ -606,6 +606,13 @@ __global__ void __launch_bounds__(256, kMinBlocks) traverse_kernel(TraverseParam
   const uint32_t lt_mask = (1u << lane) - 1u;
   const uint32_t nrays = P.ray_pref[P.njobs];
   const uint32_t refill = P.refill ? P.refill : 1u;
+  // A warp's first 32 rays are its share of the front of the list, the queue
+  // hands out the rest: thousands of warps taking their first rays from one
+  // counter at once serialise there for several microseconds, which is most
+  // of a small view's start.  Consecutive chunks go to different CTAs, so a
+  // list with fewer chunks than warps spreads over the device.  (A lane
+  // without a job has had no ray; if the warp's first chunk left it none, the
+  // list is exhausted for the warp.)
   Tally T = {0xffffffffu, 0ull, 0u};
   bool active = false, exhausted = false;
   Ray R;
@@ -615,7 +622,9 @@ __global__ void __launch_bounds__(256, kMinBlocks) traverse_kernel(TraverseParam
     if (idle && !exhausted && ((uint32_t)__popc(idle) >= refill || idle == 0xffffffffu)) {
       const uint32_t leader = __ffs(idle) - 1u, k = __popc(idle);
       uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(P.queue, k);
+      if (lane == leader)
+        base = T.j == 0xffffffffu ? 32u * ((threadIdx.x >> 5) * gridDim.x + blockIdx.x)
+                                  : gridDim.x * blockDim.x + atomicAdd(P.queue, k);
       base = __shfl_sync(0xffffffffu, base, leader);
       if (base + k >= nrays) exhausted = true;
       if (!active) {
