@@ -102,7 +102,8 @@ class BatchRenderer:
     def launches_per_run(self) -> int:
         # init, rotate, normalize, maxedge, visible, compact, prefix, raster,
         # raylist, prefix, traverse (composited: the raster replaced by two
-        # bin passes, a two-kernel scan and the tile kernel)
+        # bin passes, a two-kernel scan and the tile kernel); a batch small
+        # enough for one wave of blocks per stage runs up to three fewer
         return 11 if self.mode == _lib.MODE_REF else 15
 
     def read(self, rgb8=None, rgba=None, steps=None):

@@ -33,6 +33,8 @@ __global__ void init_jobs_kernel(const JobDev* __restrict__ jobs, uint32_t njobs
   if (j == 0) {
     queue[0] = 0;  // the traversal's ray queue
     queue[1] = 0;  // the composited mode's entry-arena cursor
+    queue[2] = 0;  // blocks done of compact_kernel (see prefix_by_last_block)
+    queue[3] = 0;  // and of raylist_kernel
   }
   if (j >= njobs) return;
   ViewCounters v;
@@ -145,42 +147,6 @@ __global__ void __launch_bounds__(256) view_normalize_kernel(const JobDev* __res
   }
 }
 
-// buildLmt's maxEdgeLength (vfRayPreComp.cc:810-836) over each view's
-// vertices.  The reference visits the 6 edges of every tet; an edge shared by
-// several tets gives the same length in each (its difference vector at most
-// changes sign), so the maximum over the mesh's distinct edges is the same
-// float, at about a seventh of the work.
-__global__ void __launch_bounds__(256) view_maxedge_kernel(const JobDev* __restrict__ jobs,
-                                                           uint32_t njobs,
-                                                           const uint32_t* __restrict__ bpref) {
-  const uint32_t j = job_of(bpref, njobs, blockIdx.x);
-  const JobDev& J = jobs[j];
-  const uint32_t lb = blockIdx.x - bpref[j], nb = bpref[j + 1] - bpref[j];
-  // the rounded square root is monotone, so the largest rounded length is
-  // the rounded root of the largest squared length: one root per thread
-  float best_sq = 0.0f;
-  for (uint32_t e = lb * blockDim.x + threadIdx.x; e < J.nEdges; e += nb * blockDim.x) {
-    const uint2 ed = __ldg(J.edges + e);
-    if (id_bad(ed.x, J.nV) || id_bad(ed.y, J.nV)) {
-      atomicOr(&J.ctr->status, kDevRange);
-      continue;
-    }
-    const float4 a = J.vview[ed.x], b = J.vview[ed.y];
-    const float e0 = fsub(a.x, b.x), e1 = fsub(a.y, b.y), e2 = fsub(a.z, b.z);
-    const float sq = fadd(fadd(fmul(e0, e0), fmul(e1, e1)), fmul(e2, e2));
-    if (sq > best_sq) best_sq = sq;
-  }
-  float best = __fsqrt_rn(best_sq);
-  __shared__ float s_best[8];
-  best = warp_max(best);
-  if ((threadIdx.x & 31u) == 0) s_best[threadIdx.x >> 5] = best;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (uint32_t i = 1; i < (blockDim.x >> 5); ++i) best = fmaxf(best, s_best[i]);
-    atomicMax(&J.ctr->maxedge_bits, __float_as_uint(best));
-  }
-}
-
 // Keys of the 6 edges of every tet, (min id << 32) | max id, to be sorted and
 // made unique into the mesh's distinct edges.
 __global__ void __launch_bounds__(256) edge_keys_kernel(const uint4* __restrict__ tet, uint32_t nT,
@@ -199,11 +165,63 @@ __global__ void __launch_bounds__(256) edge_keys_kernel(const uint4* __restrict_
 
 // ------------------------------------------------------------ stage (a)
 
+// buildLmt's maxEdgeLength (vfRayPreComp.cc:810-836) over each view's
+// vertices.  The reference visits the 6 edges of every tet; an edge shared by
+// several tets gives the same length in each (its difference vector at most
+// changes sign), so the maximum over the mesh's distinct edges is the same
+// float, at about a seventh of the work.
+__device__ __forceinline__ void view_maxedge(const JobDev* __restrict__ jobs, uint32_t njobs,
+                                             const uint32_t* __restrict__ bpref, uint32_t block) {
+  const uint32_t j = job_of(bpref, njobs, block);
+  const JobDev& J = jobs[j];
+  const uint32_t lb = block - bpref[j], nb = bpref[j + 1] - bpref[j];
+  // the rounded square root is monotone, so the largest rounded length is
+  // the rounded root of the largest squared length: one root per thread
+  float best_sq = 0.0f;
+  for (uint32_t e = lb * blockDim.x + threadIdx.x; e < J.nEdges; e += nb * blockDim.x) {
+    const uint2 ed = __ldg(J.edges + e);
+    if (id_bad(ed.x, J.nV) || id_bad(ed.y, J.nV)) {
+      atomicOr(&J.ctr->status, kDevRange);
+      continue;
+    }
+    const float4 a = J.vview[ed.x], b = J.vview[ed.y];
+    const float e0 = fsub(a.x, b.x), e1 = fsub(a.y, b.y), e2 = fsub(a.z, b.z);
+    const float sq = fadd(fadd(fmul(e0, e0), fmul(e1, e1)), fmul(e2, e2));
+    if (sq > best_sq) best_sq = sq;
+  }
+  float best = __fsqrt_rn(best_sq);
+  __shared__ float s_best[32];
+  best = warp_max(best);
+  if ((threadIdx.x & 31u) == 0) s_best[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (uint32_t i = 1; i < (blockDim.x >> 5); ++i) best = fmaxf(best, s_best[i]);
+    atomicMax(&J.ctr->maxedge_bits, __float_as_uint(best));
+  }
+}
+
+__global__ void __launch_bounds__(256) view_maxedge_kernel(const JobDev* __restrict__ jobs,
+                                                           uint32_t njobs,
+                                                           const uint32_t* __restrict__ bpref) {
+  view_maxedge(jobs, njobs, bpref, blockIdx.x);
+}
+
 // findVisibleFaces (vfRayKernelCPU.cc:51-132), one thread per external face;
-// each block of 1024 faces belongs to one job (bpref: blocks per job).
+// each block of 1024 faces belongs to one job (bpref: blocks per job).  The
+// blocks after the ext_blocks first take the views' longest edge (epref: edge
+// blocks per job): both need only the view's vertices, and where the blocks
+// of both fit the device at once, one launch saves 5 us of a small view's
+// chain.  A larger grid runs view_maxedge_kernel, whose smaller blocks gather
+// edges faster (32 views of the carved 64^3 mesh: 0.26 ms less).
 __global__ void __launch_bounds__(1024) visible_kernel(const JobDev* __restrict__ jobs,
                                                        uint32_t njobs,
-                                                       const uint32_t* __restrict__ bpref) {
+                                                       const uint32_t* __restrict__ bpref,
+                                                       uint32_t ext_blocks,
+                                                       const uint32_t* __restrict__ epref) {
+  if (blockIdx.x >= ext_blocks) {
+    view_maxedge(jobs, njobs, epref, blockIdx.x - ext_blocks);
+    return;
+  }
   const uint32_t j = job_of(bpref, njobs, blockIdx.x);
   const JobDev& J = jobs[j];
   const uint32_t lb = blockIdx.x - bpref[j];
@@ -237,12 +255,87 @@ __global__ void __launch_bounds__(1024) visible_kernel(const JobDev* __restrict_
   if (threadIdx.x == 0) J.blk[lb] = (uint32_t)cnt;
 }
 
+// Exclusive prefix of a per-job device count (0: visible faces, 1: rays) into
+// out[0..njobs], by one block of 256 or 1024 threads.
+__device__ __forceinline__ void prefix_block(const JobDev* __restrict__ jobs, uint32_t njobs,
+                                             int which, uint32_t* __restrict__ out) {
+  __shared__ uint32_t s[32];
+  __shared__ uint32_t s_carry;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) s_carry = 0;
+  __syncthreads();
+  for (uint32_t base = 0; base < njobs; base += blockDim.x) {
+    const uint32_t j = base + threadIdx.x;
+    uint32_t v = 0;
+    if (j < njobs) {
+      const ViewCounters* c = jobs[j].ctr;
+      v = __ldcg(which == 0 ? &c->nvis : &c->nrays);  // other blocks' writes
+    }
+    uint32_t x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= (uint32_t)o) x += y;
+    }
+    if (lane == 31) s[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+      const uint32_t c = lane < (blockDim.x >> 5) ? s[lane] : 0u;
+      uint32_t z = c;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, z, o);
+        if (lane >= (uint32_t)o) z += y;
+      }
+      s[lane] = z - c;
+    }
+    __syncthreads();
+    const uint32_t carry = s_carry;
+    if (j < njobs) out[j] = carry + s[warp] + x - v;
+    __syncthreads();
+    if (threadIdx.x == blockDim.x - 1) s_carry = carry + s[warp] + x;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[njobs] = s_carry;
+}
+
+// Called at the end of a kernel that produces a per-job count: the block that
+// finishes last makes its prefix, which saves a one-block launch (3 us of a
+// small view's chain each).  done counts the finished blocks (zeroed by
+// init_jobs_kernel); every block's counts are fenced before its arrival.
+// done is null where the grid is more than one wave of blocks: there the
+// blocks' fences, each waiting for its block's stores, cost more than the
+// launch (a 1024x768 view gains nothing, 32 views at 512^2 lose 0.04 ms).
+__device__ __forceinline__ void prefix_by_last_block(const JobDev* __restrict__ jobs,
+                                                     uint32_t njobs, int which,
+                                                     uint32_t* __restrict__ out,
+                                                     uint32_t* __restrict__ done) {
+  __shared__ bool s_last;
+  if (!done) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(done, 1u) == gridDim.x - 1u;
+  }
+  __syncthreads();
+  if (s_last) {
+    __threadfence();
+    prefix_block(jobs, njobs, which, out);
+    if (threadIdx.x == 0) *done = 0;
+  }
+}
+
+__global__ void __launch_bounds__(1024) prefix_kernel(const JobDev* __restrict__ jobs, uint32_t njobs,
+                                                      int which, uint32_t* __restrict__ out) {
+  prefix_block(jobs, njobs, which, out);
+}
+
 // Ordered compaction (main.cc:93-138, vfRay.cu:355-388): a block's offset is
 // the sum of the counts of the job's blocks before it; inside the block,
 // warp ballots and a warp-count prefix place each face at its rank.
 __global__ void __launch_bounds__(1024) compact_kernel(const JobDev* __restrict__ jobs,
                                                        uint32_t njobs,
-                                                       const uint32_t* __restrict__ bpref) {
+                                                       const uint32_t* __restrict__ bpref,
+                                                       uint32_t* __restrict__ vis_pref,
+                                                       uint32_t* __restrict__ done) {
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_base;
   const uint32_t j = job_of(bpref, njobs, blockIdx.x);
@@ -279,48 +372,7 @@ __global__ void __launch_bounds__(1024) compact_kernel(const JobDev* __restrict_
   }
   __syncthreads();
   if (vis) J.vis_ext[s_base + s_warp[warp] + __popc(m & ((1u << lane) - 1u))] = e;
-}
-
-// Exclusive prefix of a per-job device count (0: visible faces, 1: rays,
-// 2: entry-list entries) into out[0..njobs]; one block.
-__global__ void __launch_bounds__(1024) prefix_kernel(const JobDev* __restrict__ jobs, uint32_t njobs,
-                                                      int which, uint32_t* __restrict__ out) {
-  __shared__ uint32_t s[32];
-  __shared__ uint32_t s_carry;
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_carry = 0;
-  __syncthreads();
-  for (uint32_t base = 0; base < njobs; base += blockDim.x) {
-    const uint32_t j = base + threadIdx.x;
-    uint32_t v = 0;
-    if (j < njobs) {
-      const ViewCounters* c = jobs[j].ctr;
-      v = which == 0 ? c->nvis : (which == 1 ? c->nrays : c->nentries);
-    }
-    uint32_t x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= (uint32_t)o) x += y;
-    }
-    if (lane == 31) s[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-      const uint32_t c = lane < (blockDim.x >> 5) ? s[lane] : 0u;
-      uint32_t z = c;
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, z, o);
-        if (lane >= (uint32_t)o) z += y;
-      }
-      s[lane] = z - c;
-    }
-    __syncthreads();
-    const uint32_t carry = s_carry;
-    if (j < njobs) out[j] = carry + s[warp] + x - v;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) s_carry = carry + s[warp] + x;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[njobs] = s_carry;
+  prefix_by_last_block(jobs, njobs, 0, vis_pref, done);
 }
 
 // ------------------------------------------------------------ stage (b)
@@ -705,7 +757,8 @@ __global__ void __launch_bounds__(256) tile_kernel(const JobDev* __restrict__ jo
 // reference zero-fills its image, main.cc:194).
 __global__ void __launch_bounds__(256) raylist_kernel(const JobDev* __restrict__ jobs, uint32_t njobs,
                                                       const uint32_t* __restrict__ tpref, int mode,
-                                                      uint32_t tw) {
+                                                      uint32_t tw, uint32_t* __restrict__ ray_pref,
+                                                      uint32_t* __restrict__ done) {
   __shared__ uint32_t s_job[8], s_count[8], s_base[8];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -779,6 +832,7 @@ __global__ void __launch_bounds__(256) raylist_kernel(const JobDev* __restrict__
     if (J.rgba) J.rgba[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (J.steps) J.steps[p] = 0;
   }
+  prefix_by_last_block(jobs, njobs, 1, ray_pref, done);
 }
 
 // Exclusive scan of the batch's entry-count arena (composited mode): block

@@ -437,6 +437,13 @@ int Batch::upload(bool async) {
   return rc;
 }
 
+// Blocks of this many threads that the device holds at once (2048 threads
+// per SM): up to there a kernel's last block makes the per-job prefix itself
+// (prefix_by_last_block).
+static uint32_t one_wave(const Ctx& C, uint32_t threads) {
+  return (uint32_t)C.num_sms * (2048u / threads);
+}
+
 int Batch::enqueue_a() {
   Ctx& C = *ctx;
   const cudaStream_t st = Batch::st();
@@ -447,13 +454,16 @@ int Batch::enqueue_a() {
   if (rot_blocks) {
     view_rotate_kernel<<<rot_blocks, 256, 0, st>>>(J, njobs, P);
     view_normalize_kernel<<<rot_blocks, 256, 0, st>>>(J, njobs, P);
-    view_maxedge_kernel<<<edge_blocks, 256, 0, st>>>(J, njobs, P + n1);
   }
-  if (ext_blocks) {
-    visible_kernel<<<ext_blocks, fb, 0, st>>>(J, njobs, P + 2 * n1);
-    compact_kernel<<<ext_blocks, fb, 0, st>>>(J, njobs, P + 2 * n1);
-  }
-  prefix_kernel<<<1, fb, 0, st>>>(J, njobs, 0, vis_pref());
+  const bool both = ext_blocks + edge_blocks <= one_wave(C, fb);
+  if (edge_blocks && !both) view_maxedge_kernel<<<edge_blocks, 256, 0, st>>>(J, njobs, P + n1);
+  if (const uint32_t blocks = ext_blocks + (both ? edge_blocks : 0u))
+    visible_kernel<<<blocks, fb, 0, st>>>(J, njobs, P + 2 * n1, ext_blocks, P + n1);
+  const bool fold = ext_blocks && ext_blocks <= one_wave(C, fb);
+  if (ext_blocks)
+    compact_kernel<<<ext_blocks, fb, 0, st>>>(J, njobs, P + 2 * n1, vis_pref(),
+                                              fold ? queue() + 2 : nullptr);
+  if (!fold) prefix_kernel<<<1, fb, 0, st>>>(J, njobs, 0, vis_pref());
   return C.cuda(cudaGetLastError(), "stage (a) launch");
 }
 
@@ -487,8 +497,11 @@ int Batch::enqueue_b() {
           J, njobs, ps, tile_off.as<uint32_t>(), bins.as<uint32_t>(), bcap, ent.as<uint4>(),
           (uint32_t)std::min<size_t>(ent_cap, 0xffffffffu), queue() + 1);
   }
-  if (tiles) raylist_kernel<<<cdiv(tiles, 8), 256, 0, st>>>(J, njobs, P + 3 * n1, mode, tile_w);
-  prefix_kernel<<<1, fb, 0, st>>>(J, njobs, 1, ray_pref());
+  // (every image has a tile: W and H are at least 2)
+  const bool fold = cdiv(tiles, 8) <= one_wave(C, 256);
+  raylist_kernel<<<cdiv(tiles, 8), 256, 0, st>>>(J, njobs, P + 3 * n1, mode, tile_w, ray_pref(),
+                                                 fold ? queue() + 3 : nullptr);
+  if (!fold) prefix_kernel<<<1, fb, 0, st>>>(J, njobs, 1, ray_pref());
   return C.cuda(cudaGetLastError(), "stage (b) launch");
 }
 
