@@ -609,17 +609,34 @@ __global__ void __launch_bounds__(256) tile_kernel(const JobDev* __restrict__ jo
     const JobDev& J = jobs[j];
     const uint32_t lt = g - tpref[j], W = J.W, H = J.H;
     const uint32_t tpx = (W + kTile - 1) / kTile;
-    const uint32_t px = (lt % tpx) * kTile + (tid % kTile), py = (lt / tpx) * kTile + tid / kTile;
+    // a warp's pixels are an 8 x 4 block of the tile
+    const uint32_t wx = (lt % tpx) * kTile + (warp & 1u) * 8u, wy = (lt / tpx) * kTile + (warp >> 1) * 4u;
+    const uint32_t px = wx + (lane & 7u), py = wy + (lane >> 3);
     const bool live = px < W && py < H;
     const double rW = __drcp_rn((double)(float)(W - 1u)), rH = __drcp_rn((double)(float)(H - 1u));
     const float ox = obj_coord_r(px, rW), oy = obj_coord_r(py, rH);
     const uint32_t b0 = min(tile_off[g], bin_cap), b1 = min(tile_off[g + 1], bin_cap);
     auto covers = [&](const TileFace& f) {
-      return px >= f.box.x && px <= min(f.box.z, W - 1) && py >= f.box.y &&
-             py <= min(f.box.w, H - 1) && entry_inside(f.E, ox, oy) && [&] {
+      return px >= f.box.x && px <= f.box.z && py >= f.box.y && py <= f.box.w &&
+             entry_inside(f.E, ox, oy) && [&] {
                const float sp = plane_eval(ox, oy, f.sx, f.sy, f.sz);
                return (sp >= 0.0f) && (sp <= 1.0f);
              }();
+    };
+    // which of the staged faces 32 w .. 32 w + 31 have a box that meets the
+    // warp's pixels, one face per lane: the others need no test at any pixel
+    // (an 801x600 view of the carved 48^3 mesh: 45 -> 38 us against testing
+    // every face at every pixel; with 16 x 2 pixels per warp fewer faces drop
+    // out.  Selecting each next entry over the mask in shared memory, with no
+    // insertion in the arena, was slower: 41 us)
+    auto meets = [&](uint32_t w, uint32_t m) {
+      const uint32_t k = 32u * w + lane;
+      bool ov = false;
+      if (k < m) {
+        const uint4 b = F[k].box;
+        ov = b.x <= wx + 7u && b.z >= wx && b.y <= wy + 3u && b.w >= wy;
+      }
+      return __ballot_sync(0xffffffffu, ov);
     };
     auto stage = [&](uint32_t c) {  // faces c .. c+255 of the bin into shared memory
       __syncthreads();
@@ -636,6 +653,8 @@ __global__ void __launch_bounds__(256) tile_kernel(const JobDev* __restrict__ jo
         const float4 p0 = pl[0], p1 = pl[1], p2 = pl[2];
         TileFace f;
         f.box = bad ? make_uint4(1u, 1u, 0u, 0u) : J.bbox[i];  // bad: covers nothing
+        f.box.z = min(f.box.z, W - 1);
+        f.box.w = min(f.box.w, H - 1);
         f.E = entry_edges(make_float4(p1.z, p1.w, 0.0f, 0.0f), make_float4(p2.x, p2.y, 0.0f, 0.0f),
                           make_float4(p2.z, p2.w, 0.0f, 0.0f));
         f.zx = p0.x;
@@ -660,14 +679,15 @@ __global__ void __launch_bounds__(256) tile_kernel(const JobDev* __restrict__ jo
     uint32_t cov[8];
     uint32_t count = 0;
     for (uint32_t c = b0; c < b1; c += 256) {
-      const uint32_t staged = stage(c);  // every thread: stage() synchronises the block
-      const uint32_t m = live ? staged : 0u;
+      const uint32_t m = stage(c);  // every thread: stage() synchronises the block
 #pragma unroll
       for (uint32_t w = 0; w < 8; ++w) {  // w is a constant after unrolling: cov stays in registers
         uint32_t bits = 0;
-        const uint32_t kn = min(m, 32u * w + 32u);
-        for (uint32_t k = 32u * w; k < kn; ++k)
-          if (covers(F[k])) bits |= 1u << (k & 31u);
+        if (32u * w < m)
+          for (uint32_t todo = meets(w, m); todo; todo &= todo - 1u) {
+            const uint32_t k = (uint32_t)__ffs(todo) - 1u;
+            if (live && covers(F[32u * w + k])) bits |= 1u << k;
+          }
         cov[w] = bits;
         count += __popc(bits);
       }
@@ -736,9 +756,11 @@ __global__ void __launch_bounds__(256) tile_kernel(const JobDev* __restrict__ jo
     } else {
       for (uint32_t c = b0; c < b1; c += 256) {
         const uint32_t m = stage(c);
-        if (live && fits && count)
-          for (uint32_t k = 0; k < m; ++k)
-            if (covers(F[k])) insert(F[k]);
+        for (uint32_t w = 0; 32u * w < m; ++w)
+          for (uint32_t todo = meets(w, m); todo; todo &= todo - 1u) {
+            const TileFace& f = F[32u * w + (uint32_t)__ffs(todo) - 1u];
+            if (live && fits && count && covers(f)) insert(f);
+          }
       }
     }
   }
