@@ -58,6 +58,10 @@ struct Mesh {
   // with a model-view (its maxEdgeLength is recomputed per view)
   uint2* edges = nullptr;
   uint32_t nEdges = 0;
+  // the edges within kLongEdge of the longest come first (nLong of them, 0 if
+  // they are not few), the longest edge and the largest vertex coordinate
+  uint32_t nLong = 0;
+  float edgeMax = 0, vertMax = 0;
   size_t bytes = 0;
   ~Mesh() {
     if (edges) cudaFree(edges);

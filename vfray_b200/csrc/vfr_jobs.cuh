@@ -147,6 +147,21 @@ __global__ void __launch_bounds__(256) view_normalize_kernel(const JobDev* __res
   }
 }
 
+// A mesh edge's squared length.
+__host__ __device__ __forceinline__ float edge_sq(const float4* vert, uint2 e) {
+  const float4 a = vert[e.x], b = vert[e.y];
+  const float x = a.x - b.x, y = a.y - b.y, z = a.z - b.z;
+  return x * x + y * y + z * z;
+}
+struct LongEdge {
+  const float4* vert;
+  float least;  // squared length
+  __host__ __device__ bool operator()(unsigned long long k) const {
+    // the two ids as they lie in memory (little-endian: the high word second)
+    return edge_sq(vert, make_uint2((uint32_t)k, (uint32_t)(k >> 32))) >= least;
+  }
+};
+
 // Keys of the 6 edges of every tet, (min id << 32) | max id, to be sorted and
 // made unique into the mesh's distinct edges.
 __global__ void __launch_bounds__(256) edge_keys_kernel(const uint4* __restrict__ tet, uint32_t nT,
@@ -163,6 +178,26 @@ __global__ void __launch_bounds__(256) edge_keys_kernel(const uint4* __restrict_
   }
 }
 
+// The longest edge's squared length and the largest coordinate of the
+// vertices, as float bits.
+__global__ void __launch_bounds__(256) edge_extent_kernel(const uint2* __restrict__ edges, uint32_t n,
+                                                          const float4* __restrict__ vert,
+                                                          uint32_t nV, uint32_t* __restrict__ out) {
+  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  float sq = 0.0f, co = 0.0f;
+  for (uint32_t i = i0; i < n; i += step) sq = fmaxf(sq, edge_sq(vert, edges[i]));
+  for (uint32_t i = i0; i < nV; i += step) {
+    const float4 v = vert[i];
+    co = fmaxf(co, fmaxf(fabsf(v.x), fmaxf(fabsf(v.y), fabsf(v.z))));
+  }
+  sq = warp_max(sq);
+  co = warp_max(co);
+  if ((threadIdx.x & 31u) == 0) {
+    atomicMax(out, __float_as_uint(sq));
+    atomicMax(out + 1, __float_as_uint(co));
+  }
+}
+
 // ------------------------------------------------------------ stage (a)
 
 // buildLmt's maxEdgeLength (vfRayPreComp.cc:810-836) over each view's
@@ -170,15 +205,51 @@ __global__ void __launch_bounds__(256) edge_keys_kernel(const uint4* __restrict_
 // several tets gives the same length in each (its difference vector at most
 // changes sign), so the maximum over the mesh's distinct edges is the same
 // float, at about a seventh of the work.
+//
+// Where the model-view is a similarity (a rotation, with any scale), the
+// view's longest edge is one of the mesh's long ones: a view keeps all
+// lengths in proportion up to its rounding, so only the edges within
+// kLongEdge of the mesh's longest, which the edge list starts with, can be
+// the view's longest.  long_edges_suffice bounds how far a length can be off
+// its proportion.  64 views of the carved 64^3 mesh: 315 -> 11
+// us.
+constexpr float kLongEdge = 1.0f - 0x1p-9f;  // of the squared length
+__device__ __forceinline__ bool long_edges_suffice(const JobDev& J) {
+  if (!J.nLong) return false;
+  const double u = 0x1p-24;
+  const float4 m[3] = {J.m0, J.m1, J.m2};
+  double g[6], s2 = 0, reach = 0, half = 0;
+#pragma unroll
+  for (int a = 0, q = 0; a < 3; ++a) {
+#pragma unroll
+    for (int b = a; b < 3; ++b, ++q)
+      g[q] = (double)m[a].x * m[b].x + (double)m[a].y * m[b].y + (double)m[a].z * m[b].z;
+    // rotated coordinates are within 5 u of this (three products, four sums)
+    reach = fmax(reach, ((double)fabsf(m[a].x) + fabsf(m[a].y) + fabsf(m[a].z)) * J.vertMax + fabsf(m[a].w));
+    half = fmax(half, 0.5 * ((double)ord2f(J.ctr->mm[4 + a]) - ord2f(J.ctr->mm[a])));
+  }
+  s2 = (g[0] + g[3] + g[5]) / 3.0;
+  // M M^T = s2 (1 + E): squared lengths keep proportion within 1 +- 3 eta
+  const double eta = fmax(fmax(fmax(fabs(g[0] - s2), fabs(g[3] - s2)), fabs(g[5] - s2)),
+                          fmax(fmax(fabs(g[1]), fabs(g[2])), fabs(g[4]))) / s2;
+  // normalised: scaled by 1 / half, coordinates at most 1; each end of an
+  // edge is off by rounding in its 3 coordinates, its length by 8 u besides
+  const double length = sqrt(s2) * J.edgeMax / half;
+  const double eps = 16.0 * u + 3.5 * (10.0 * u * reach / half + 4.0 * u) / length;
+  return 8.0 * eta + 2.5 * eps < 0x1p-11;  // false for a NaN too; half the margin of kLongEdge
+}
+
 __device__ __forceinline__ void view_maxedge(const JobDev* __restrict__ jobs, uint32_t njobs,
                                              const uint32_t* __restrict__ bpref, uint32_t block) {
   const uint32_t j = job_of(bpref, njobs, block);
   const JobDev& J = jobs[j];
   const uint32_t lb = block - bpref[j], nb = bpref[j + 1] - bpref[j];
+  const uint32_t n = long_edges_suffice(J) ? J.nLong : J.nEdges;
+  if (lb * blockDim.x >= n) return;
   // the rounded square root is monotone, so the largest rounded length is
   // the rounded root of the largest squared length: one root per thread
   float best_sq = 0.0f;
-  for (uint32_t e = lb * blockDim.x + threadIdx.x; e < J.nEdges; e += nb * blockDim.x) {
+  for (uint32_t e = lb * blockDim.x + threadIdx.x; e < n; e += nb * blockDim.x) {
     const uint2 ed = __ldg(J.edges + e);
     if (id_bad(ed.x, J.nV) || id_bad(ed.y, J.nV)) {
       atomicOr(&J.ctr->status, kDevRange);

@@ -9,6 +9,7 @@
 // CUDA graph.  A single view is a batch of one job.
 #include <cuda_runtime.h>
 
+#include <cub/device/device_partition.cuh>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_select.cuh>
 
@@ -166,7 +167,7 @@ int Ctx::mesh_edges(Mesh* m, cudaStream_t st) {
   unsigned long long *keys = nullptr, *sorted = nullptr, *uniq = nullptr;
   unsigned long long* count = nullptr;
   void* tmp = nullptr;
-  size_t tmp_sort = 0, tmp_uniq = 0;
+  size_t tmp_sort = 0, tmp_uniq = 0, tmp_part = 0;
   int rc = cuda(cudaMalloc(&keys, n * 8), "edge keys");
   if (!rc) rc = cuda(cudaMalloc(&sorted, n * 8), "edge keys");
   if (!rc) rc = cuda(cudaMalloc(&uniq, n * 8), "edge keys");
@@ -174,7 +175,8 @@ int Ctx::mesh_edges(Mesh* m, cudaStream_t st) {
   if (!rc) {
     cub::DeviceRadixSort::SortKeys(nullptr, tmp_sort, keys, sorted, n, 0, 32 + bits, st);
     cub::DeviceSelect::Unique(nullptr, tmp_uniq, sorted, uniq, count, n, st);
-    rc = cuda(cudaMalloc(&tmp, std::max(tmp_sort, tmp_uniq)), "edge sort scratch");
+    cub::DevicePartition::If(nullptr, tmp_part, uniq, sorted, count, n, LongEdge{m->vert, 0.0f}, st);
+    rc = cuda(cudaMalloc(&tmp, std::max(std::max(tmp_sort, tmp_uniq), tmp_part)), "edge sort scratch");
   }
   if (!rc) {
     edge_keys_kernel<<<cdiv(m->nT, 256), 256, 0, st>>>(m->tet, m->nT, keys);
@@ -187,8 +189,24 @@ int Ctx::mesh_edges(Mesh* m, cudaStream_t st) {
     rc = cuda(cudaMemcpyAsync(&ne, count, sizeof(ne), cudaMemcpyDeviceToHost, st), "edge count");
   if (!rc) rc = cuda(cudaStreamSynchronize(st), "edge build");
   if (!rc) rc = cuda(cudaMalloc(&m->edges, sizeof(uint2) * std::max<size_t>(ne, 1)), "edges");
-  if (!rc) rc = cuda(cudaMemcpyAsync(m->edges, uniq, sizeof(uint2) * ne, cudaMemcpyDeviceToDevice, st),
-                     "edges");
+  // the longest edges first (view_maxedge); count is free again by now
+  uint32_t extent[2] = {0, 0};
+  if (!rc) rc = cuda(cudaMemsetAsync(count, 0, sizeof(unsigned long long), st), "edge extent");
+  if (!rc) {
+    edge_extent_kernel<<<2 * num_sms, 256, 0, st>>>(reinterpret_cast<const uint2*>(uniq), (uint32_t)ne,
+                                                    m->vert, m->nV, reinterpret_cast<uint32_t*>(count));
+    rc = cuda(cudaMemcpyAsync(extent, count, sizeof extent, cudaMemcpyDeviceToHost, st), "edge extent");
+  }
+  if (!rc) rc = cuda(cudaStreamSynchronize(st), "edge build");
+  float sq, co;
+  std::memcpy(&sq, &extent[0], sizeof sq);
+  std::memcpy(&co, &extent[1], sizeof co);
+  unsigned long long nl = 0;
+  if (!rc && ne)
+    rc = cuda(cub::DevicePartition::If(tmp, tmp_part, uniq, reinterpret_cast<unsigned long long*>(m->edges),
+                                       count, ne, LongEdge{m->vert, sq * kLongEdge}, st),
+              "edge partition");
+  if (!rc) rc = cuda(cudaMemcpyAsync(&nl, count, sizeof(nl), cudaMemcpyDeviceToHost, st), "edge count");
   if (!rc) rc = cuda(cudaStreamSynchronize(st), "edge build");
   for (void* p : {(void*)keys, (void*)sorted, (void*)uniq, (void*)count, tmp})
     if (p) cudaFree(p);
@@ -198,6 +216,10 @@ int Ctx::mesh_edges(Mesh* m, cudaStream_t st) {
     return rc;
   }
   m->nEdges = (uint32_t)ne;
+  // lengths too near zero or infinity, or too many long edges: not listed
+  m->nLong = sq > 0x1p-60f && sq < 0x1p60f && nl <= ne / 4 ? (uint32_t)nl : 0u;
+  m->edgeMax = std::sqrt(sq) * (1.0f - 0x1p-20f);
+  m->vertMax = co;
   m->bytes += sizeof(uint2) * ne;
   return VFR_OK;
 }
@@ -263,14 +285,13 @@ int Batch::layout(const std::vector<JobSpec>& s, int m, bool own_outputs) {
   uint32_t* pt = px + (njobs + 1);
   uint32_t* ps = pt + (njobs + 1);  // composited: 16 x 16 screen tiles
   size_t nv_mv = 0, next = 0, nblk = 0, pix = 0;
+  uint64_t all_edges = 0;  // of the jobs with a model-view
   for (uint32_t j = 0; j < njobs; ++j) {
     Mesh* mesh = C.mesh(s[j].mesh);
     if (!mesh) return C.fail(VFR_ERR_STATE, "unknown mesh id in job");
     const JobSpec& q = s[j];
     if (q.W < 2 || q.H < 2 || (uint64_t)q.W * q.H > (1ull << 28))
       return C.fail(VFR_ERR_INVALID, "image size out of range");
-    const uint32_t rb =
-        q.use_mv ? std::max<uint32_t>(1, std::min<uint32_t>(cdiv(mesh->nV, 1024), 2 * C.num_sms)) : 0;
     if (q.use_mv && !mesh->edges) {
       // built once per mesh (allocates and waits): a server builds them all
       // before its launch starts
@@ -278,8 +299,19 @@ int Batch::layout(const std::vector<JobSpec>& s, int m, bool own_outputs) {
       const int rc = C.mesh_edges(mesh, st());
       if (rc) return rc;
     }
+    all_edges += q.use_mv ? mesh->nEdges : 0;
+  }
+  for (uint32_t j = 0; j < njobs; ++j) {
+    const Mesh* mesh = C.mesh(s[j].mesh);
+    const JobSpec& q = s[j];
+    const uint32_t rb =
+        q.use_mv ? std::max<uint32_t>(1, std::min<uint32_t>(cdiv(mesh->nV, 1024), 2 * C.num_sms)) : 0;
+    // a share of one wave of blocks by the mesh's edges: most blocks have
+    // nothing to do (view_maxedge)
     const uint32_t eb =
-        q.use_mv ? std::max<uint32_t>(1, std::min<uint32_t>(cdiv(mesh->nEdges, 1024), 4 * C.num_sms))
+        q.use_mv ? std::max<uint32_t>(1, std::min<uint32_t>(cdiv(mesh->nEdges, 1024),
+                                                            cdiv(8ull * C.num_sms * mesh->nEdges,
+                                                                 std::max<uint64_t>(all_edges, 1))))
                  : 0;
     const uint32_t xb = cdiv(mesh->nExt, fb);
     const uint32_t tl = cdiv(q.W, C.tune.tile_w) * cdiv(q.H, 32 / C.tune.tile_w);
@@ -350,6 +382,9 @@ int Batch::layout(const std::vector<JobSpec>& s, int m, bool own_outputs) {
     J.tet = mesh->tet;
     J.edges = mesh->edges;
     J.nEdges = mesh->nEdges;
+    J.nLong = mesh->nLong;
+    J.edgeMax = mesh->edgeMax;
+    J.vertMax = mesh->vertMax;
     J.walk = mesh->walk;
     J.vert_in = mesh->vert;
     J.extf = mesh->extf;

@@ -32,7 +32,8 @@ struct __align__(16) JobDev {
   float4 m0, m1, m2;         // rows of the model-view (use_mv)
   const uint4* tet;          // mesh
   const uint2* edges;        // the mesh's distinct edges (jobs with a model-view)
-  uint32_t nEdges;
+  uint32_t nEdges, nLong;    // the first nLong: the mesh's long edges (0: not listed)
+  float edgeMax, vertMax;    // the mesh's longest edge and largest vertex coordinate
   const WalkRec* walk;
   const float4* vert_in;     // the mesh's (normalised) vertices
   const uint2* extf;
