@@ -23,6 +23,20 @@ __device__ __forceinline__ uint32_t job_of(const uint32_t* __restrict__ pref, ui
   return lo;
 }
 
+// The same for one g per warp, 32 steps of the search at a time: called by the
+// whole warp.
+__device__ __forceinline__ uint32_t job_of_warp(const uint32_t* __restrict__ pref, uint32_t n, uint32_t g) {
+  uint32_t lo = 0;
+  while (n > 1) {  // the job is one of lo .. lo + n - 1, and pref[lo] <= g
+    const uint32_t step = (n + 31u) / 32u, at = step * (threadIdx.x & 31u);
+    const uint32_t below = __ballot_sync(0xffffffffu, at < n && __ldg(pref + lo + at) <= g);
+    const uint32_t skip = step * (uint32_t)(__popc(below) - 1);
+    lo += skip;
+    n = min(step, n - skip);
+  }
+  return lo;
+}
+
 __device__ __forceinline__ float job_maxedge(const JobDev& J) {
   return J.use_mv ? __uint_as_float(J.ctr->maxedge_bits) : J.maxEdge_in;
 }
@@ -882,7 +896,7 @@ __global__ void __launch_bounds__(256) raylist_kernel(const JobDev* __restrict__
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const bool any = g < tpref[njobs];  // else a warp past the last tile: no pixels
-  const uint32_t j = any ? job_of(tpref, njobs, g) : njobs - 1u;
+  const uint32_t j = any ? job_of_warp(tpref, njobs, g) : njobs - 1u;
   const JobDev& J = jobs[j];
   const uint32_t tile = any ? g - tpref[j] : 0u;
   const uint32_t th = 32u / tw;
@@ -910,7 +924,8 @@ __global__ void __launch_bounds__(256) raylist_kernel(const JobDev* __restrict__
       if (has) {
         const float4* pl = J.planes + kPlaneStride * (size_t)w;
         const float4 p0 = pl[0], p1 = pl[1];
-        const float ox = obj_coord(x, J.W), oy = obj_coord(y, J.H);
+        const float ox = obj_coord_r(x, __drcp_rn((double)(float)(J.W - 1u))),
+                    oy = obj_coord_r(y, __drcp_rn((double)(float)(J.H - 1u)));
         const uint2 tf = J.extf[w];
         rs.tf = (tf.x << 2) | (tf.y & 3u);
         rs.zp = __float_as_uint(plane_eval(ox, oy, p0.x, p0.y, p0.z));
