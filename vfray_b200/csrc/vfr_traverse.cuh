@@ -229,6 +229,16 @@ __device__ __forceinline__ WalkRec ldg_walk(const WalkRec* w, uint32_t t) {
   return r;
 }
 
+// The four vertices of a tet in the slots, rotated by its entry face f.
+__device__ __forceinline__ void set_vertices(Ray& R, uint4 id, uint32_t f) {
+  const uint32_t ident = identity_map();
+  set_vtx(vtx_at(ident, R.low, 1), __ldg(R.vert + sel4(id, f)));
+  set_vtx(vtx_at(ident, R.low, 2), __ldg(R.vert + sel4(id, (f + 1) & 3u)));
+  set_vtx(vtx_at(ident, R.low, 3), __ldg(R.vert + sel4(id, (f + 2) & 3u)));
+  set_vtx(vtx_at(ident, R.low, 0), __ldg(R.vert + sel4(id, (f + 3) & 3u)));
+  R.map = ident;
+}
+
 // Start a segment in tet t through its face f, with entry depth zp and the
 // back colour's transfer-function entry cbi (:256-279).  False (checked build
 // only): the tet or one of its vertex ids is out of range, and nothing was
@@ -242,12 +252,7 @@ __device__ __forceinline__ bool begin_segment_at(const SharedTables& S, const Jo
   if (id_bad(id.x, J.nV) || id_bad(id.y, J.nV) || id_bad(id.z, J.nV) || id_bad(id.w, J.nV))
     return false;
   R.w = ldg_walk(R.walk, t);
-  const uint32_t ident = identity_map();
-  set_vtx(vtx_at(ident, R.low, 1), __ldg(R.vert + sel4(id, f)));
-  set_vtx(vtx_at(ident, R.low, 2), __ldg(R.vert + sel4(id, (f + 1) & 3u)));
-  set_vtx(vtx_at(ident, R.low, 3), __ldg(R.vert + sel4(id, (f + 2) & 3u)));
-  set_vtx(vtx_at(ident, R.low, 0), __ldg(R.vert + sel4(id, (f + 3) & 3u)));
-  R.map = ident;
+  set_vertices(R, id, f);
   R.zp = zp;
   R.lastZ = zp;
   R.cb = S.tf[cbi];
@@ -300,7 +305,9 @@ __device__ __forceinline__ void finish_pixel(const JobDev& J, const Ray& R) {
   if (J.steps) J.steps[R.p] = R.iters;
 }
 
-enum StepResult : uint32_t { kContinue = 0, kSegmentEnd = 1, kCycle = 2, kCap = 3, kRange = 4 };
+enum StepResult : uint32_t {
+  kContinue = 0, kSegmentEnd = 1, kReload = 2, kCycle = 3, kCap = 4, kRange = 5
+};
 
 // The step cap of a ray of this job: the option, or 4 nT + 64 (a walk that
 // repeats no state has at most 4 nT iterations).
@@ -434,7 +441,6 @@ __device__ __forceinline__ uint32_t step(const TraverseParams& P, const SharedTa
   const bool xo = (ex & 1u) != 0u, xh = (ex & 2u) != 0u;
   const uint32_t tn = xh ? (xo ? R.w.n.w : R.w.n.z) : (xo ? R.w.n.y : R.w.n.x);
   const uint32_t q = xh ? (xo ? R.w.q.w : R.w.q.z) : (xo ? R.w.q.y : R.w.q.x);
-  const bool leaving = (tn == R.t);
   // both loads of the step, issued before the plane solve that hides them,
   // whatever the exit: tn and the vertex word are valid ids for every face
   // (a boundary face's record names the tet itself and vertex 0; the mesh's
@@ -493,7 +499,10 @@ __device__ __forceinline__ uint32_t step(const TraverseParams& P, const SharedTa
     R.lastZ = zn;
     R.cb = front;
   }
-  const bool go_on = !end && !leaving;  // :535
+  // :535 the ray leaves the mesh through a boundary face; it and a face whose
+  // vertices the records could not match by id (the walk goes on, but the
+  // caller loads the next tet's vertices first) have these two bits clear
+  const bool go_on = !end && (q & 0x60000000u) != 0u;
   // advance to tn through its face fn: the exit face's vertices in tn's order
   // (permutation code), the loaded vertex in the slot of the one left
   // behind.  Done whatever the status: once a ray's segment ends, nothing
@@ -501,26 +510,26 @@ __device__ __forceinline__ uint32_t step(const TraverseParams& P, const SharedTa
   const uint32_t fn = (q >> 27) & 3u;
   set_vtx(vtx_at(m, R.low, 0), nv);
   R.map = __byte_perm(m, 0u, perm_selector(q >> 29));
-  if (go_on && (q & 0x60000000u) == 0u) {  // kCodeMismatch: no boundary face goes on
-    // shared face not matched by vertex ids: reload the tet's vertices
-    const uint4 id = __ldg((kServe ? R.jp->tet : P.jobs[R.j].tet) + tn);
-    bad = id_bad(id.x, R.nV) || id_bad(id.y, R.nV) || id_bad(id.z, R.nV) || id_bad(id.w, R.nV);
-    if (!bad) {
-      const uint32_t ident = identity_map();
-      set_vtx(vtx_at(ident, R.low, 1), __ldg(R.vert + sel4(id, fn)));
-      set_vtx(vtx_at(ident, R.low, 2), __ldg(R.vert + sel4(id, (fn + 1) & 3u)));
-      set_vtx(vtx_at(ident, R.low, 3), __ldg(R.vert + sel4(id, (fn + 2) & 3u)));
-      set_vtx(vtx_at(ident, R.low, 0), __ldg(R.vert + sel4(id, (fn + 3) & 3u)));
-      R.map = ident;
-    }
-  }
   R.w = N;
   R.t = tn;
   R.f = fn;
   R.zp = zn;
   if (wst != kContinue) return wst;
   if (bad) return kRange;
-  return go_on ? (uint32_t)kContinue : (uint32_t)kSegmentEnd;
+  // kCodeMismatch is the only one of the two with the top bit set
+  return go_on ? (uint32_t)kContinue : kSegmentEnd + (end ? 0u : q >> 31);
+}
+
+// Rare (a face whose neighbour lists other vertices): the vertices of the tet
+// the step moved to, in the entry face's rotation.  False (checked build
+// only): an id is out of range.
+template <bool kServe>
+__device__ __forceinline__ bool reload(const TraverseParams& P, Ray& R) {
+  const uint4 id = __ldg((kServe ? R.jp->tet : P.jobs[R.j].tet) + R.t);
+  if (id_bad(id.x, R.nV) || id_bad(id.y, R.nV) || id_bad(id.z, R.nV) || id_bad(id.w, R.nV))
+    return false;
+  set_vertices(R, id, R.f);
+  return true;
 }
 
 // Start the ray of the job's local ray index `local`: its pixel, the
@@ -657,6 +666,10 @@ __global__ void __launch_bounds__(256, kMinBlocks) traverse_kernel(TraverseParam
       res = step<true>(P, S, R);
     }
     if (res == kContinue) continue;
+    if (res == kReload) {
+      if (reload<false>(P, R)) continue;
+      res = kRange;
+    }
     if (res == kSegmentEnd) {
       if (kMode == 1) {
         s_exit_z[threadIdx.x] = R.lastZ;
@@ -848,6 +861,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) serve_kernel(ServeParams SP) 
     }
     uint32_t status = 0;
     bool fin = false;
+    if (active && res == kReload) res = reload<true>(P, R) ? (uint32_t)kContinue : (uint32_t)kRange;
     if (active && res != kContinue) {
       fin = true;
       if (res == kSegmentEnd) {
