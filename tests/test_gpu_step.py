@@ -72,6 +72,18 @@ def test_extinctions_outside_the_fast_range(alpha, renderer, oracle_lib):
     _check(renderer, oracle_lib, vb.prepare(vert, tet), tf, 61, 47)
 
 
+@pytest.mark.parametrize("alpha", [2.0**30, 2.0**48, 2.0**60, 2.0**100])
+@pytest.mark.parametrize("permuted", [False, True])
+def test_power_of_two_extinctions(alpha, permuted, renderer, oracle_lib):
+    """Depth differences of a lattice seen along its axes are powers of two too,
+    so each sum's product with 32 / ln2 has zeros in the low word that holds
+    the exponential's table index."""
+    vert, tet = _lattice(4, permuted)
+    tf = synth.transfer_function(2)
+    tf[:, 3] = np.float32(alpha)
+    _check(renderer, oracle_lib, vb.prepare(vert, tet), tf, 33, 33, lmt=(1.0, 1.0, -1.0))
+
+
 @pytest.mark.parametrize("edge", [1e-35, 1e-4, 1e4, 1e20])
 def test_limits_that_do_not_fit_the_mesh(edge, renderer, oracle_lib):
     vert, tet = synth.make_mesh(5, view_seed=4)

@@ -597,8 +597,6 @@ __device__ __forceinline__ void flush(const TraverseParams& P, Tally& T) {
   T.status = 0;
 }
 
-// kMinBlocks: CTAs of 256 threads the register budget must allow per SM
-// (2: no spills; 3: 80 registers, a few spilled to L1).
 __device__ __forceinline__ void load_tables(const TraverseParams& P, SharedTables& S) {
   for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) S.tf[i] = P.tf[i];
   // 2^(-k/64) from the table of 2^(j/64), j = 0..63, scaled by a power of two
@@ -607,6 +605,8 @@ __device__ __forceinline__ void load_tables(const TraverseParams& P, SharedTable
   __syncthreads();
 }
 
+// kMinBlocks: CTAs of 256 threads the register budget must allow per SM
+// (2: no spills; 3: 80 registers, a few spilled to L1).
 template <int kMode, int kMinBlocks>
 __global__ void __launch_bounds__(256, kMinBlocks) traverse_kernel(TraverseParams P) {
   __shared__ SharedTables S;

@@ -74,7 +74,7 @@ struct TraverseParams {
   uint32_t* queue;           // work-queue head over all jobs' rays
   const float4* tf;          // 256 RGBA
   const float* psi;          // 512 x 512
-  const double* e2tab;       // 2^(j/64), j = 0..63
+  const double* e2tab;       // 2^(j/64), j = 0..63 (load_tables makes 2^(-k/64) of it)
   uint32_t step_cap;         // 0: 4 * nT + 64 of each job's mesh
   uint32_t refill;           // refill a warp's idle lanes once this many are idle
   f32x2 neg0;                // (-0.0f, -0.0f), see face_plane_pairs
