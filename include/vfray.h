@@ -325,9 +325,9 @@ VFR_API void vfr_server_destroy(vfr_server* s);
  * uint2); writes visExt_dev (visible ext-face indices in order, capacity
  * nExt) and *num_vis_dev, asynchronously on `stream` (a cudaStream_t, NULL =
  * the default stream).  Its scratch is a fixed device array inside the
- * library (32 bytes per external face for up to VFR_STATIC_MAX_EXT faces,
- * about 8 MiB, held on every GPU that loads the library until exit); larger
- * meshes get VFR_ERR_BUDGET.  The array's device address belongs to the
+ * library (a bit per external face for up to VFR_STATIC_MAX_EXT faces and a
+ * count per 256 of them, 36 KiB, held on every GPU that loads the library
+ * until exit); larger meshes get VFR_ERR_BUDGET.  The array's device address belongs to the
  * current CUDA context: a call whose stream is not capturing looks it up in
  * that context, and a call under stream capture uses the address an earlier
  * call found in the same context (VFR_ERR_STATE if none did).  Calls share
