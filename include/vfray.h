@@ -143,15 +143,16 @@ VFR_API int vfr_find_visible(vfr_ctx* ctx, int mesh_id, uint32_t* num_vis, uint3
 
 /* Stage (b): projectVisibleFaces + per-pixel entry faces (vfRayKernel.cu:171-228;
  * CPU vfRayKernelCPU.cc:136-169, main.cc:164-182).  Needs stage (a) of the
- * same mesh first.  Optional host outputs: bbox (4 per visible face:
+ * same mesh first; may be called again on the same visible faces, at any
+ * size.  Optional host outputs: bbox (4 per visible face:
  * xmin, ymin, xmax, ymax) and writer (W*H ext-face index of the face whose
  * ray the reference writes last at each pixel, -1 for none). */
 VFR_API int vfr_project(vfr_ctx* ctx, int mesh_id, uint32_t W, uint32_t H, uint32_t* bbox,
                 int32_t* writer);
 
 /* Stage (c): traversal + compositing (vfRayKernel.cu:231-852; CPU
- * vfRayKernelCPU.cc:173-566).  Needs stage (b) first.  Optional host
- * outputs: rgb8 (W*H*3), rgba (W*H*4 float: clamped colour, alpha = 1 - prod
+ * vfRayKernelCPU.cc:173-566).  Needs a stage (b) of its own first.  Optional
+ * host outputs: rgb8 (W*H*3), rgba (W*H*4 float: clamped colour, alpha = 1 - prod
  * zeta), steps (W*H tet-walk iterations of each pixel's ray). */
 VFR_API int vfr_traverse(vfr_ctx* ctx, int mesh_id, uint8_t* rgb8, float* rgba, uint32_t* steps,
                  vfr_render_stats* stats);

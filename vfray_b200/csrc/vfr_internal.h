@@ -156,6 +156,7 @@ struct Batch {
                             bool rgb8_only);
   int upload(bool async);
   int enqueue_a();
+  int enqueue_reproject();  // before another enqueue_b without an enqueue_a
   int enqueue_b();
   int enqueue_c();
   int enqueue_all() {
@@ -180,7 +181,8 @@ struct Ctx {
   float* d_psi = nullptr;
   std::vector<std::unique_ptr<Mesh>> meshes;
   Batch plain;     // the one-job batch behind the single-view calls
-  int stage = 0;   // single-view stage calls: 0 none, 1 visible done, 2 project done
+  int stage = 0;   // single-view stage calls: 0 none, 1 visible done, 2 project done,
+                   // 3 visible done and a projection begun or traversed
   cudaEvent_t ev[4] = {};
   int occ[4] = {0, 0, 0, 0};
   uint32_t step_cap = 0;

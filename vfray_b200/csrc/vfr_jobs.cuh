@@ -58,6 +58,24 @@ __global__ void init_jobs_kernel(const JobDev* __restrict__ jobs, uint32_t njobs
   *jobs[j].ctr = v;
 }
 
+// Before stages (b) and (c) run again on the visible faces of one stage (a):
+// their counts start from 0 as after init_jobs_kernel (raylist_kernel appends
+// to nrays, and the traversal's queue still holds the last run's rays).  What
+// stage (a) found stays: the visible faces, and an id out of range.
+__global__ void reproject_kernel(const JobDev* __restrict__ jobs, uint32_t njobs,
+                                 uint32_t* __restrict__ queue) {
+  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < 4u) queue[j] = 0;
+  if (j >= njobs) return;
+  ViewCounters& v = *jobs[j].ctr;
+  v.nrays = 0;
+  v.nentries = 0;
+  v.status &= kDevRange;
+  v.steps = 0;
+  v.rays_done = 0;
+  v.nbins = 0;
+}
+
 // ------------------------------------------------------------ view set-up
 
 // The view set-up kernels give each job a range of blocks (bpref: prefix of

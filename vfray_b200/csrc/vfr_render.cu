@@ -502,6 +502,11 @@ int Batch::enqueue_a() {
   return C.cuda(cudaGetLastError(), "stage (a) launch");
 }
 
+int Batch::enqueue_reproject() {
+  reproject_kernel<<<cdiv(std::max(njobs, 4u), 128), 128, 0, st()>>>(d_jobs.as<JobDev>(), njobs, queue());
+  return ctx->cuda(cudaGetLastError(), "reproject launch");
+}
+
 int Batch::enqueue_b() {
   Ctx& C = *ctx;
   const cudaStream_t st = Batch::st();
@@ -950,7 +955,10 @@ int vfr_project(vfr_ctx* c, int id, uint32_t W, uint32_t H, uint32_t* bbox, int3
     return C.fail(VFR_ERR_INVALID, "image size out of range");
   // the planes and visible list of stage (a) stay where they are: same mesh,
   // so the same arena offsets; only the pixel arenas grow
+  const bool again = C.stage > 1;
+  C.stage = 3;  // until this projection is whole, nothing may be traversed
   int rc = single(C, id, nullptr, W, H, VFR_MODE_REF, true, nullptr, nullptr, nullptr);
+  if (!rc && again) rc = C.plain.enqueue_reproject();
   if (!rc) rc = C.plain.enqueue_b();
   std::vector<vfr::ViewCounters> k;
   if (!rc) rc = C.plain.counters(k);
@@ -971,10 +979,11 @@ int vfr_traverse(vfr_ctx* c, int id, uint8_t* rgb8, float* rgba, uint32_t* steps
   vfr::Range nvtx("vfr_traverse");
   CTX_OR_FAIL(c);
   Mesh* m = C.mesh(id);
-  if (!m || C.stage < 2 || !C.plain.njobs || C.plain.specs[0].mesh != id)
+  if (!m || C.stage != 2 || !C.plain.njobs || C.plain.specs[0].mesh != id)
     return C.fail(VFR_ERR_STATE, "vfr_traverse needs vfr_project of the same mesh first");
   if (!C.d_tf) return C.fail(VFR_ERR_STATE, "tables not uploaded");
   const size_t np = (size_t)C.plain.specs[0].W * C.plain.specs[0].H;
+  C.stage = 3;  // the ray queue is consumed: project again before another traverse
   cudaEventRecord(C.ev[0], C.stream);
   int rc = C.plain.enqueue_c();
   cudaEventRecord(C.ev[1], C.stream);
@@ -988,7 +997,6 @@ int vfr_traverse(vfr_ctx* c, int id, uint8_t* rgb8, float* rgba, uint32_t* steps
     cudaEventElapsedTime(&stats->ms_traverse, C.ev[0], C.ev[1]);
     stats->ms_total = stats->ms_traverse;
   }
-  C.stage = 1;  // the ray queue is consumed; project again before another traverse
   return C.check_status(k[0].status, 0);
 }
 
