@@ -23,7 +23,9 @@ Workloads (seeded synthetic meshes, transfer function and cameras):
            carving, 85.6 M after: 4.1 GB of tet and walk records, far beyond
            L2); building the mesh on the host takes about two minutes.
 Every workload renders with the reference's own psi table
-(psiGammaTable512.h, shipped with the library).
+(psiGammaTable512.h, converted beside the library where the build finds the
+reference sources, or the file $VFRAY_PSI_TABLE names); without either, with
+the library's generated table.  ``config.psi_table`` says which.
 
 Timing: W untimed warm-up steps, then K steps, each bracketed by CUDA events
 on the render stream after an L2 flush (a 256 MiB write) that is not timed;
@@ -149,10 +151,26 @@ def workload_spec(name, views=64):
     return sp
 
 
+REFERENCE_PSI = "the reference's psiGammaTable512.h"
+
+
+def bench_psi_table():
+    """(table, what it is): the library's default table, the reference's own,
+    where it is present, else the generated one, which differs from it in a
+    near-diagonal band only."""
+    import vfray_b200 as vb
+
+    try:
+        table = vb.reference_psi_table()
+    except vb.VfrError:
+        return vb.psi_table(), "generated (vfr_psi_table; the reference's table is not present)"
+    name = os.environ.get("VFRAY_PSI_TABLE")
+    return table, f"the file $VFRAY_PSI_TABLE names ({os.path.basename(name)})" if name else REFERENCE_PSI
+
+
 def prepare_ours(sp):
     """The load sequence of the reference driver (normalizeVertices,
-    buildCon, buildExtF, buildLmt) through this library, and its default psi
-    table (the reference's own)."""
+    buildCon, buildExtF, buildLmt) through this library, and the psi table."""
     import vfray_b200 as vb
 
     meshes = []
@@ -160,7 +178,8 @@ def prepare_ours(sp):
         p = vb.prepare(m["vert"], m["tet"])
         p["n"] = m["n"]
         meshes.append(p)
-    return dict(sp, meshes=meshes, psi=vb.reference_psi_table())
+    psi, psi_name = bench_psi_table()
+    return dict(sp, meshes=meshes, psi=psi, psi_name=psi_name)
 
 
 def mesh_info(meshes):
@@ -176,7 +195,7 @@ def workload_config(wl, rays_per_step, mode):
             "rays_per_step": int(rays_per_step),
             "mode": ("composited (every entry segment, depth-ordered)" if mode == "composited"
                      else "reference (last visible face wins)"),
-            "psi_table": "the reference's psiGammaTable512.h", "l2": L2_NOTE}
+            "psi_table": wl["psi_name"], "l2": L2_NOTE}
 
 
 def max_over_ranks(values, dist, device):
@@ -418,6 +437,10 @@ def cpu_baseline(wl, seconds):
     """The reference's CPU kernels on this host over a bounded sample of the
     workload's jobs (in order): a third of the time single-threaded, as the
     reference is written, the rest on all host cores."""
+    import oracle
+
+    if not oracle.ref_available("fast"):
+        return {"unavailable": "reference CPU build (oracle/_ref) missing"}
     meshes = [dict(p, n_ext=int(p["extf"].shape[0])) for p in wl["meshes"]]
     run = RefRunner(meshes, wl["jobs"], wl["tf"])
     nthreads = os.cpu_count() or 1
@@ -467,7 +490,7 @@ def run_reference(args, rank):
     sp = workload_spec(name, args.views)
     with tempfile.TemporaryDirectory() as tmp:
         meshes = reference_meshes_from_files(sp, tmp)
-    wl = dict(sp, meshes=meshes)
+    wl = dict(sp, meshes=meshes, psi_name=REFERENCE_PSI)
     run = RefRunner(meshes, sp["jobs"], meshes[0]["tf"])
     nthreads = os.cpu_count() or 1
     nj = len(sp["jobs"])
@@ -1000,7 +1023,7 @@ def main():
     out, wl = res
     if not args.no_cpu_baseline and world == 1:
         out["cpu_baseline"] = cpu_baseline(wl, args.cpu_seconds)
-        if args.mode == "composited":
+        if args.mode == "composited" and "sample" in out["cpu_baseline"]:
             out["cpu_baseline"]["sample"] += (" (its own last-visible-face render: the reference "
                                               "has no composited mode)")
     if dist:
