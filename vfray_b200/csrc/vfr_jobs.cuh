@@ -187,18 +187,21 @@ __global__ void __launch_bounds__(256) view_normalize_kernel(const JobDev* __res
   }
 }
 
-// A mesh edge's squared length.
-__host__ __device__ __forceinline__ float edge_sq(const float4* vert, uint2 e) {
+// A mesh edge's squared length; infinite where an id is out of range (checked
+// build), so that no edges are listed as long and every view meets this one.
+__host__ __device__ __forceinline__ float edge_sq(const float4* vert, uint32_t nV, uint2 e) {
+  if (id_bad(e.x, nV) || id_bad(e.y, nV)) return INFINITY;
   const float4 a = vert[e.x], b = vert[e.y];
   const float x = a.x - b.x, y = a.y - b.y, z = a.z - b.z;
   return x * x + y * y + z * z;
 }
 struct LongEdge {
   const float4* vert;
+  uint32_t nV;
   float least;  // squared length
   __host__ __device__ bool operator()(unsigned long long k) const {
     // the two ids as they lie in memory (little-endian: the high word second)
-    return edge_sq(vert, make_uint2((uint32_t)k, (uint32_t)(k >> 32))) >= least;
+    return edge_sq(vert, nV, make_uint2((uint32_t)k, (uint32_t)(k >> 32))) >= least;
   }
 };
 
@@ -225,7 +228,7 @@ __global__ void __launch_bounds__(256) edge_extent_kernel(const uint2* __restric
                                                           uint32_t nV, uint32_t* __restrict__ out) {
   const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
   float sq = 0.0f, co = 0.0f;
-  for (uint32_t i = i0; i < n; i += step) sq = fmaxf(sq, edge_sq(vert, edges[i]));
+  for (uint32_t i = i0; i < n; i += step) sq = fmaxf(sq, edge_sq(vert, nV, edges[i]));
   for (uint32_t i = i0; i < nV; i += step) {
     const float4 v = vert[i];
     co = fmaxf(co, fmaxf(fabsf(v.x), fmaxf(fabsf(v.y), fabsf(v.z))));

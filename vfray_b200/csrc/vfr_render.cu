@@ -175,7 +175,7 @@ int Ctx::mesh_edges(Mesh* m, cudaStream_t st) {
   if (!rc) {
     cub::DeviceRadixSort::SortKeys(nullptr, tmp_sort, keys, sorted, n, 0, 32 + bits, st);
     cub::DeviceSelect::Unique(nullptr, tmp_uniq, sorted, uniq, count, n, st);
-    cub::DevicePartition::If(nullptr, tmp_part, uniq, sorted, count, n, LongEdge{m->vert, 0.0f}, st);
+    cub::DevicePartition::If(nullptr, tmp_part, uniq, sorted, count, n, LongEdge{m->vert, m->nV, 0.0f}, st);
     rc = cuda(cudaMalloc(&tmp, std::max(std::max(tmp_sort, tmp_uniq), tmp_part)), "edge sort scratch");
   }
   if (!rc) {
@@ -204,7 +204,7 @@ int Ctx::mesh_edges(Mesh* m, cudaStream_t st) {
   unsigned long long nl = 0;
   if (!rc && ne)
     rc = cuda(cub::DevicePartition::If(tmp, tmp_part, uniq, reinterpret_cast<unsigned long long*>(m->edges),
-                                       count, ne, LongEdge{m->vert, sq * kLongEdge}, st),
+                                       count, ne, LongEdge{m->vert, m->nV, sq * kLongEdge}, st),
               "edge partition");
   if (!rc) rc = cuda(cudaMemcpyAsync(&nl, count, sizeof(nl), cudaMemcpyDeviceToHost, st), "edge count");
   if (!rc) rc = cuda(cudaStreamSynchronize(st), "edge build");
