@@ -622,7 +622,15 @@ def run_ours(args, rank, world, dist):
         runner.run()
 
     step = batched_step if args.form == "batched" else plain_step
-    launches_per_step = runner.launches_per_run() if args.form == "batched" else 11 * nj
+    if args.form == "batched":
+        launches_per_step = runner.launches_per_run()
+    else:  # a view alone launches what a batch of it does
+        launches_per_step = 0
+        for j in jobs:
+            one = vbatch.BatchRenderer(r, [j], mode=mode)
+            one.prepare()
+            launches_per_step += one.launches_per_run()
+            one.close()
 
     def timed(fn, K, Wu, profile=False):
         for _ in range(Wu):

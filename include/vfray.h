@@ -244,6 +244,10 @@ typedef struct {
   float ms;  /* stages (b) + (c) of the batch with these knobs */
 } vfr_tuning;
 VFR_API int vfr_batch_autotune(vfr_batch* b, int reps, vfr_tuning* out);
+/* Kernels that one run of the batch launches, as it was last captured or run
+ * (0 before that): small batches fold some of the chain's launches into
+ * others. */
+VFR_API int vfr_batch_launches(vfr_batch* b, uint32_t* count);
 /* Device bytes of the batch's scratch arenas. */
 VFR_API int vfr_batch_scratch_bytes(vfr_batch* b, uint64_t* bytes);
 

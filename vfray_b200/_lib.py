@@ -143,6 +143,7 @@ SIGNATURES = {
     "vfr_batch_set_stream": (_i, [_vp, _vp]),
     "vfr_batch_set_cameras": (_i, [_vp, _vp, _u32]),
     "vfr_batch_autotune": (_i, [_vp, _i, C.POINTER(Tuning)]),
+    "vfr_batch_launches": (_i, [_vp, C.POINTER(C.c_uint32)]),
     "vfr_batch_scratch_bytes": (_i, [_vp, C.POINTER(C.c_uint64)]),
     "vfr_server_create": (_i, [_vp, C.c_uint64, _u32, C.POINTER(_vp)]),
     "vfr_server_submit": (_i, [_vp, C.POINTER(Request), C.POINTER(C.c_uint64)]),

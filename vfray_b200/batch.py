@@ -100,11 +100,16 @@ class BatchRenderer:
         return int(b.value)
 
     def launches_per_run(self) -> int:
-        # init, rotate, normalize, maxedge, visible, compact, prefix, raster,
-        # raylist, prefix, traverse (composited: the raster replaced by two
-        # bin passes, a two-kernel scan and the tile kernel); a batch small
-        # enough for one wave of blocks per stage runs up to three fewer
-        return 11 if self.mode == _lib.MODE_REF else 15
+        """Kernels one run launches, as the batch was last captured or run (0
+        before that): init, rotate, normalize, maxedge, visible, compact,
+        prefix, raster, raylist, prefix, traverse (composited: the raster
+        replaced by two bin passes, a two-kernel scan and the tile kernel).
+        Jobs without a model-view skip the three of the view set-up, and a
+        batch small enough for one wave of blocks per stage folds up to three
+        into others."""
+        n = C.c_uint32()
+        check(self.lib.vfr_batch_launches(self.h, C.byref(n)), self.r.h, "vfr_batch_launches")
+        return int(n.value)
 
     def read(self, rgb8=None, rgba=None, steps=None):
         """Copy every job's outputs (concatenated in job order) into host

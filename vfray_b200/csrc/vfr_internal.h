@@ -124,6 +124,7 @@ struct Batch {
   Buf tile_cnt, tile_off, tile_cur, bins;  // composited: faces binned by screen tile
   Buf out_rgb8, out_rgba, out_steps;      // outputs owned by the batch (host-output calls)
   size_t ent_cap = 0, bin_cap = 0;  // composited: entry and bin capacities (0: sized at layout)
+  uint32_t launches[3] = {0, 0, 0};  // kernels of stages (a), (b), (c) as last enqueued
   cudaGraphExec_t exec = nullptr;
   cudaStream_t stream = nullptr;  // null: the context's stream
   cudaStream_t st() const;

@@ -499,6 +499,8 @@ int Batch::enqueue_a() {
     compact_kernel<<<ext_blocks, fb, 0, st>>>(J, njobs, P + 2 * n1, vis_pref(),
                                               fold ? queue() + 2 : nullptr);
   if (!fold) prefix_kernel<<<1, fb, 0, st>>>(J, njobs, 0, vis_pref());
+  launches[0] = 1u + (rot_blocks ? 2u : 0u) + (edge_blocks && !both ? 1u : 0u) +
+                (ext_blocks || (both && edge_blocks) ? 1u : 0u) + (ext_blocks ? 1u : 0u) + (fold ? 0u : 1u);
   return C.cuda(cudaGetLastError(), "stage (a) launch");
 }
 
@@ -542,6 +544,7 @@ int Batch::enqueue_b() {
   raylist_kernel<<<cdiv(tiles, 8), 256, 0, st>>>(J, njobs, P + 3 * n1, mode, tile_w, ray_pref(),
                                                  fold ? queue() + 3 : nullptr);
   if (!fold) prefix_kernel<<<1, fb, 0, st>>>(J, njobs, 1, ray_pref());
+  launches[1] = (mode == VFR_MODE_REF ? 1u : 4u + (stiles ? 1u : 0u)) + 1u + (fold ? 0u : 1u);
   return C.cuda(cudaGetLastError(), "stage (b) launch");
 }
 
@@ -560,6 +563,7 @@ int Batch::enqueue_c() {
   P.neg0 = 0x8000000080000000ull;
   const int blocks = C.num_sms * C.traverse_blocks_per_sm(mode);
   void* args[] = {&P};
+  launches[2] = 1u;
   return C.cuda(cudaLaunchKernel(C.traverse_fn(mode, C.tune.variant), dim3(blocks), dim3(256), args,
                                  0, st()),
                 "stage (c) launch");
@@ -1379,6 +1383,12 @@ int vfr_batch_set_stream(vfr_batch* b, void* stream) {
   // work already enqueued on the old stream is not ordered with the new one
   if (int rc = C.cuda(cudaStreamSynchronize(b->b.st()), "batch stream switch")) return rc;
   b->b.stream = static_cast<cudaStream_t>(stream);
+  return VFR_OK;
+}
+
+int vfr_batch_launches(vfr_batch* b, uint32_t* count) {
+  if (!b || !count) return VFR_ERR_INVALID;
+  *count = b->b.launches[0] + b->b.launches[1] + b->b.launches[2];
   return VFR_OK;
 }
 
