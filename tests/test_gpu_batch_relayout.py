@@ -1,0 +1,55 @@
+"""A batch whose job list changes: a list that is refused leaves the batch, its
+captured graph and its outputs as they were."""
+import numpy as np
+import pytest
+
+import vfray_b200 as vb
+from vfray_b200 import batch as vbatch
+from vfray_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def scene(renderer):
+    renderer.upload_tables(synth.transfer_function(2), vb.psi_table())
+    ids = []
+    for n, carved in ((9, True), (6, False)):
+        p = vb.prepare(*synth.make_mesh(n, carved=carved, view_seed=None))
+        ids.append(renderer.upload_mesh(p["vert"], p["tet"], p["con"], p["extf"], p["lmt"]))
+    yield ids
+    for m in ids:
+        renderer.release_mesh(m)
+
+
+def _read(B, jobs):
+    rgb = np.empty(sum(W * H for _, _, W, H in jobs) * 3, np.uint8)
+    B.read(rgb8=rgb)
+    at = np.cumsum([0] + [W * H * 3 for _, _, W, H in jobs])
+    return [rgb[at[k]:at[k + 1]].reshape(H, W, 3) for k, (_, _, W, H) in enumerate(jobs)]
+
+
+def _lists(ids):
+    v = synth.orbit_views(8, seed=3)
+    return [[(ids[k % 2], v[k], 48 + 8 * k, 40) for k in range(8)]]
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_refused_list_leaves_the_batch_as_it_was(graph, renderer, scene):
+    jobs = _lists(scene)[0]
+    bad = [(scene[0], None, 1, 64)]
+    B = vbatch.BatchRenderer(renderer, jobs, graph=graph)
+    try:
+        B.prepare()
+        B.run()
+        want = _read(B, jobs)
+        for refused in (bad, jobs * 4 + bad, [(12345, None, 32, 32)] * 40):
+            with pytest.raises(vb.VfrError):
+                B.set_jobs(refused)
+            B.run()
+            B.stats()
+            assert all(np.array_equal(a, b) for a, b in zip(_read(B, jobs), want))
+    finally:
+        B.close()
+    with pytest.raises(vb.VfrError):
+        vbatch.BatchRenderer(renderer, bad)

@@ -53,11 +53,13 @@ class BatchRenderer:
 
     def set_jobs(self, jobs):
         js = [j if isinstance(j, Job) else job(j[0], j[2], j[3], mv=j[1]) for j in jobs]
-        self.jobs = js  # keeps each job's output tensors alive (job())
         arr = (Job * len(js))(*js)
-        self._arr = arr
         check(self.lib.vfr_batch_set_jobs(self.h, arr, len(js), self.mode), self.r.h,
               "vfr_batch_set_jobs")
+        # a refused list leaves the batch, and the output tensors of its jobs,
+        # as they were
+        self.jobs = js  # keeps each job's output tensors alive (job())
+        self._arr = arr
         self.captured = False
 
     def autotune(self, reps: int = 2) -> dict:

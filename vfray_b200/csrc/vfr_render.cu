@@ -273,6 +273,30 @@ size_t Batch::arena_bytes(Ctx& C, const std::vector<JobSpec>& s, int mode, uint3
 
 int Batch::layout(const std::vector<JobSpec>& s, int m, bool own_outputs) {
   Ctx& C = *ctx;
+  // what is refused is refused before anything changes: the batch's host and
+  // device tables stay those of its last layout, which can still run
+  uint64_t all_edges = 0, all_pix = 0, all_ext = 0;  // edges: of the jobs with a model-view
+  for (const JobSpec& q : s) {
+    Mesh* mesh = C.mesh(q.mesh);
+    if (!mesh) return C.fail(VFR_ERR_STATE, "unknown mesh id in job");
+    if (q.W < 2 || q.H < 2 || (uint64_t)q.W * q.H > (1ull << 28))
+      return C.fail(VFR_ERR_INVALID, "image size out of range");
+    all_pix += (uint64_t)q.W * q.H;
+    all_ext += mesh->nExt;
+  }
+  if (all_pix > 0xffffffffull || all_ext > 0xffffffffull)
+    return C.fail(VFR_ERR_BUDGET, "batch too large");
+  for (const JobSpec& q : s) {
+    Mesh* mesh = C.mesh(q.mesh);
+    if (q.use_mv && !mesh->edges) {
+      // built once per mesh (allocates and waits): a server builds them all
+      // before its launch starts
+      if (arena) return C.fail(VFR_ERR_STATE, "mesh edges missing for an arena layout");
+      const int rc = C.mesh_edges(mesh, st());
+      if (rc) return rc;
+    }
+    all_edges += q.use_mv ? mesh->nEdges : 0;
+  }
   specs = s;
   mode = m;
   tile_w = C.tune.tile_w;
@@ -285,22 +309,6 @@ int Batch::layout(const std::vector<JobSpec>& s, int m, bool own_outputs) {
   uint32_t* pt = px + (njobs + 1);
   uint32_t* ps = pt + (njobs + 1);  // composited: 16 x 16 screen tiles
   size_t nv_mv = 0, next = 0, nblk = 0, pix = 0;
-  uint64_t all_edges = 0;  // of the jobs with a model-view
-  for (uint32_t j = 0; j < njobs; ++j) {
-    Mesh* mesh = C.mesh(s[j].mesh);
-    if (!mesh) return C.fail(VFR_ERR_STATE, "unknown mesh id in job");
-    const JobSpec& q = s[j];
-    if (q.W < 2 || q.H < 2 || (uint64_t)q.W * q.H > (1ull << 28))
-      return C.fail(VFR_ERR_INVALID, "image size out of range");
-    if (q.use_mv && !mesh->edges) {
-      // built once per mesh (allocates and waits): a server builds them all
-      // before its launch starts
-      if (arena) return C.fail(VFR_ERR_STATE, "mesh edges missing for an arena layout");
-      const int rc = C.mesh_edges(mesh, st());
-      if (rc) return rc;
-    }
-    all_edges += q.use_mv ? mesh->nEdges : 0;
-  }
   for (uint32_t j = 0; j < njobs; ++j) {
     const Mesh* mesh = C.mesh(s[j].mesh);
     const JobSpec& q = s[j];
@@ -332,7 +340,6 @@ int Batch::layout(const std::vector<JobSpec>& s, int m, bool own_outputs) {
   stiles = ps[njobs];
   pixels = pix;
   ext_total = next;
-  if (pix > 0xffffffffull || next > 0xffffffffull) return C.fail(VFR_ERR_BUDGET, "batch too large");
   const size_t old_sig = (size_t)vview.p ^ (size_t)planes.p ^ (size_t)winner.p ^ (size_t)rays.p ^
                          (size_t)ent.p ^ (size_t)d_jobs.p;
   int rc = place(d_jobs, sizeof(JobDev) * njobs, "job table");
@@ -364,7 +371,11 @@ int Batch::layout(const std::vector<JobSpec>& s, int m, bool own_outputs) {
     if (!rc && !rgb8_only) rc = place(out_rgba, sizeof(float4) * pix, "rgba outputs");
     if (!rc && !rgb8_only) rc = place(out_steps, sizeof(uint32_t) * pix, "steps outputs");
   }
-  if (rc) return rc;
+  if (rc) {  // a buffer is missing: nothing to run until another layout
+    njobs = 0;
+    drop_graph();
+    return rc;
+  }
   const size_t new_sig = (size_t)vview.p ^ (size_t)planes.p ^ (size_t)winner.p ^ (size_t)rays.p ^
                          (size_t)ent.p ^ (size_t)d_jobs.p;
   if (new_sig != old_sig) drop_graph();
