@@ -1,4 +1,5 @@
-"""A batch whose job list changes: a list that is refused leaves the batch, its
+"""A batch whose job list changes: another list runs as that list whether or
+not it is captured again, and a list that is refused leaves the batch, its
 captured graph and its outputs as they were."""
 import numpy as np
 import pytest
@@ -31,7 +32,34 @@ def _read(B, jobs):
 
 def _lists(ids):
     v = synth.orbit_views(8, seed=3)
-    return [[(ids[k % 2], v[k], 48 + 8 * k, 40) for k in range(8)]]
+    return [
+        [(ids[k % 2], v[k], 48 + 8 * k, 40) for k in range(8)],
+        [(ids[1], v[1], 130, 70), (ids[0], None, 33, 65)],  # fewer, other sizes
+        [(ids[0], v[k % 8], 40, 40) for k in range(12)],
+        [(ids[0], v[(k + 3) % 8], 40, 40) for k in range(12)],  # other cameras only
+        [(ids[0], v[k % 8], 40, 39) for k in range(12)],  # the same tiles, other pixels
+    ]
+
+
+@pytest.mark.parametrize("mode", [vb.MODE_REF, vb.MODE_COMPOSITED])
+@pytest.mark.parametrize("capture", ["first", "each", "never"])
+def test_another_list_of_jobs(mode, capture, renderer, scene):
+    lists = _lists(scene)
+    B = vbatch.BatchRenderer(renderer, lists[0], mode=mode)
+    try:
+        for k, jobs in enumerate(lists + lists[::-1]):
+            if k:
+                B.set_jobs(jobs)
+            if capture == "each" or (capture == "first" and k == 0):
+                B.prepare()
+            B.run()
+            B.stats()
+            got = _read(B, jobs)
+            for g, (mid, mv, W, H) in zip(got, jobs):
+                want = renderer.render(mid, W, H, mv=mv, mode=mode, rgba=False, steps=False)["rgb8"]
+                assert np.array_equal(g, want), (k, W, H)
+    finally:
+        B.close()
 
 
 @pytest.mark.parametrize("graph", [False, True])

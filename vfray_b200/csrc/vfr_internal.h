@@ -126,6 +126,7 @@ struct Batch {
   size_t ent_cap = 0, bin_cap = 0;  // composited: entry and bin capacities (0: sized at layout)
   uint32_t launches[3] = {0, 0, 0};  // kernels of stages (a), (b), (c) as last enqueued
   cudaGraphExec_t exec = nullptr;
+  std::vector<uint64_t> graph_key;  // what the last layout's launches are made of
   cudaStream_t stream = nullptr;  // null: the context's stream
   cudaStream_t st() const;
   // pinned staging for the per-call upload of a one-job batch

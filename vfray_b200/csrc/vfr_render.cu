@@ -340,8 +340,6 @@ int Batch::layout(const std::vector<JobSpec>& s, int m, bool own_outputs) {
   stiles = ps[njobs];
   pixels = pix;
   ext_total = next;
-  const size_t old_sig = (size_t)vview.p ^ (size_t)planes.p ^ (size_t)winner.p ^ (size_t)rays.p ^
-                         (size_t)ent.p ^ (size_t)d_jobs.p;
   int rc = place(d_jobs, sizeof(JobDev) * njobs, "job table");
   if (!rc) rc = place(d_pref, sizeof(uint32_t) * pref.size(), "job prefixes");
   if (!rc) rc = place(d_dev_pref, sizeof(uint32_t) * (2 * (size_t)(njobs + 1) + 4), "device prefixes");
@@ -376,9 +374,15 @@ int Batch::layout(const std::vector<JobSpec>& s, int m, bool own_outputs) {
     drop_graph();
     return rc;
   }
-  const size_t new_sig = (size_t)vview.p ^ (size_t)planes.p ^ (size_t)winner.p ^ (size_t)rays.p ^
-                         (size_t)ent.p ^ (size_t)d_jobs.p;
-  if (new_sig != old_sig) drop_graph();
+  // a captured graph holds the launches' grids and arguments; what the job
+  // table holds is read on each run
+  std::vector<uint64_t> key = {njobs, (uint64_t)mode, tile_w, pix, ent_cap, bin_cap};
+  for (const Buf* b : {&d_jobs, &d_pref, &d_dev_pref, &winner, &tile_cnt, &tile_off, &tile_cur, &scan,
+                       &bins, &ent})
+    key.push_back((uint64_t)(size_t)b->p);
+  key.insert(key.end(), pref.begin(), pref.end());
+  if (key != graph_key) drop_graph();
+  graph_key = std::move(key);
   scratch_bytes = vview.cap + planes.cap + blk.cap + vis.cap + bbox.cap + rays.cap + winner.cap +
                   ent_cnt.cap + ent_off.cap + tile_cnt.cap + tile_off.cap + tile_cur.cap + bins.cap +
                   ent.cap + scan.cap + d_ctr.cap;
