@@ -974,7 +974,7 @@ def run_served(args):
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
             "data": "synthetic (seeded meshes, TF, cameras and arrivals)",
             "config": {"workload": "served", "desc": wl["desc"], "meshes": mesh_info(wl["meshes"]),
-                       "budget_bytes": budget, "rates": results},
+                       "psi_table": wl["psi_name"], "budget_bytes": budget, "rates": results},
             "served_at_saturation_over_plain": round(best["mrays_s"] / plain_mrays, 3),
             "plain_per_view_same_mix": {"value": round(plain_mrays, 2), "unit": "Mrays/s",
                                         "requests": len(mix),
