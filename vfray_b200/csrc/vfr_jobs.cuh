@@ -541,9 +541,8 @@ __global__ void __launch_bounds__(256, 4) raster_kernel(const JobDev* __restrict
   // loads and sets up one of them (plane, box, entry edges: 32 independent
   // load chains in flight instead of one), then the warp covers the faces one
   // after another with the setup broadcast from the lane that made it
-  // (1.25 -> 0.83 ms for 64 views at 512^2 against one warp per face; the
-  // register bound of 4 CTAs per SM spills 20 bytes and beats the unbounded
-  // 70 registers at 3 CTAs).  Covering is serial in a warp, so where there
+  // (1.25 -> 0.83 ms for 64 views at 512^2 against one warp per face, 0.60
+  // with the broadcast below; 56 registers, 4 CTAs per SM).  Covering is serial in a warp, so where there
   // are fewer than 32 faces per launched warp -- a single view has a few
   // thousand to a few ten thousand -- each warp takes only its share.  The
   // broadcasts are shared-memory reads of one record (five wide loads; 22

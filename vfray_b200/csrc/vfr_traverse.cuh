@@ -159,7 +159,8 @@ static __device__ __noinline__ uint32_t exit_face_exact(uint32_t map, uint32_t l
 // the ray is strictly inside it, and -A_3 lies in one of the three sectors
 // the A_j cut the plane into.  sure says that all this holds (NaN and
 // infinite coordinates fail it); about one step in 2^13 is not sure and
-// takes the exact tests.
+// takes the exact tests (every step of a lattice seen along its axes, where
+// two vertices of each tet lie in front of one another).
 //
 // 40 instructions instead of 66 for three exact tests, with the six
 // products shared between the candidates.
@@ -192,7 +193,7 @@ __device__ __forceinline__ uint32_t exit_face(uint32_t map, uint32_t low, float 
 // Composited mode: the pixel's entry list (first, count), the next entry to
 // take and the depth where the last segment left the mesh, in shared memory:
 // only a segment's end reads them, and the step needs the registers (spills
-// 46 -> 22 bytes at 3 CTAs per SM).
+// 46 -> 22 bytes at 3 CTAs per SM then; now 16).
 __shared__ uint32_t s_ea[256], s_en[256], s_de[256];
 __shared__ float s_exit_z[256];
 
@@ -620,7 +621,7 @@ __device__ __forceinline__ void load_tables(const TraverseParams& P, SharedTable
 }
 
 // kMinBlocks: CTAs of 256 threads the register budget must allow per SM
-// (2: no spills; 3: 80 registers, a few spilled to L1).
+// (2: no spills; 3: 80 registers, 16 to 24 bytes spilled to L1).
 template <int kMode, int kMinBlocks>
 __global__ void __launch_bounds__(256, kMinBlocks) traverse_kernel(TraverseParams P) {
   __shared__ SharedTables S;
